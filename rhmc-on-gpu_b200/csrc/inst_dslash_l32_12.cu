@@ -1,0 +1,8 @@
+// inst_dslash_l32_12.cu -- instantiation of dslash_run.cuh for the L32_12 link format.
+#include "dslash_run.cuh"
+
+namespace rhmc {
+
+template cudaError_t dslash_run<L32_12>(rhmc_ctx *, const L32_12 &, int, void *, const void *, size_t, int, const void *, double, double);
+
+}  // namespace rhmc

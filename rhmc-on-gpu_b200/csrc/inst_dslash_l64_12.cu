@@ -1,0 +1,8 @@
+// inst_dslash_l64_12.cu -- instantiation of dslash_run.cuh for the L64_12 link format.
+#include "dslash_run.cuh"
+
+namespace rhmc {
+
+template cudaError_t dslash_run<L64_12>(rhmc_ctx *, const L64_12 &, int, void *, const void *, size_t, int, const void *, double, double);
+
+}  // namespace rhmc
