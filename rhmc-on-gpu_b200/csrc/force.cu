@@ -7,7 +7,7 @@
 //   fermion_force_kernel TA(U F_f) with F_f the outer products of fermionforce
 //                        (lib/Action/fermionforce.cc:46-104): even x: sum a_i h_i(x+mu) (x) x_i(x)^*,
 //                        odd x: -sum a_i x_i(x+mu) (x) h_i(x)^*, h_i = Doe x_i (with its 1/2).
-// gauge_force_kernel runs one thread per site for a fixed mu (the block index modulo 4);
+// gauge_force_kernel runs one thread per site and mu (a warp per mu);
 // fermion_force_kernel one thread per link, mu fastest inside a site (the four links of a site
 // share the site's spinor loads through L1).  All shifted solutions of all right-hand sides are summed in registers,
 // so the 18-real force matrix never goes to HBM (the reference GPU code read-modify-writes an
@@ -38,13 +38,14 @@ __device__ __forceinline__ int hidx(const Geom &g, const Site &s) { return half_
 
 // S_mu(x) = sum_{nu != mu} [ U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag
 //                          + U_nu(x+mu-nu)^dag U_mu(x-nu)^dag U_nu(x-nu) ]
-// Each staple is formed row by row (one row of the two-link product live at a time), with the
-// same operation order per element as a full product followed by a sum.
+// Each staple is formed row by row (one row of the two-link product live at a time) and its last
+// product accumulates into S, so every complex multiply-add is four FMAs: 108 per 3x3 product.
 __device__ M3 staple_sum(const Geom &g, const double2 *__restrict__ U, int mu, int p, const Site &s)
 {
     const int Vh = g.Vh, q = 1 - p;
     const Site xpm = shifted(g, s, mu, +1);
     const int kxpm = hidx(g, xpm), kx = hidx(g, s);
+    const C zero = mk<double>(0.0, 0.0);
     M3 S = m3_zero();
 #pragma unroll 1
     for (int nu = 0; nu < 4; nu++) {
@@ -56,21 +57,13 @@ __device__ M3 staple_sum(const Geom &g, const double2 *__restrict__ U, int mu, i
             const M3 Cm = load_link64(U, Vh, nu, p, kx);
 #pragma unroll
             for (int i = 0; i < 3; i++) {
-                C t[3];
+                C t[3];  // row i of A B^dag
 #pragma unroll
-                for (int l = 0; l < 3; l++) {
-                    C v = A.e[i][0] * conj(B.e[l][0]);
-                    v = v + A.e[i][1] * conj(B.e[l][1]);
-                    v = v + A.e[i][2] * conj(B.e[l][2]);
-                    t[l] = v;
-                }
+                for (int l = 0; l < 3; l++)
+                    t[l] = cmaddc(A.e[i][2], B.e[l][2], cmaddc(A.e[i][1], B.e[l][1], cmaddc(A.e[i][0], B.e[l][0], zero)));
 #pragma unroll
-                for (int j = 0; j < 3; j++) {
-                    C v = t[0] * conj(Cm.e[j][0]);
-                    v = v + t[1] * conj(Cm.e[j][1]);
-                    v = v + t[2] * conj(Cm.e[j][2]);
-                    S.e[i][j] = S.e[i][j] + v;
-                }
+                for (int j = 0; j < 3; j++)
+                    S.e[i][j] = cmaddc(t[2], Cm.e[j][2], cmaddc(t[1], Cm.e[j][1], cmaddc(t[0], Cm.e[j][0], S.e[i][j])));
             }
         }
         {
@@ -82,19 +75,11 @@ __device__ M3 staple_sum(const Geom &g, const double2 *__restrict__ U, int mu, i
             for (int i = 0; i < 3; i++) {
                 C col[3];  // column i of A B
 #pragma unroll
-                for (int l = 0; l < 3; l++) {
-                    C v = A.e[l][0] * B.e[0][i];
-                    v = cmadd(A.e[l][1], B.e[1][i], v);
-                    v = cmadd(A.e[l][2], B.e[2][i], v);
-                    col[l] = v;
-                }
+                for (int l = 0; l < 3; l++)
+                    col[l] = cmadd(A.e[l][2], B.e[2][i], cmadd(A.e[l][1], B.e[1][i], cmadd(A.e[l][0], B.e[0][i], zero)));
 #pragma unroll
-                for (int j = 0; j < 3; j++) {
-                    C v = conj(col[0]) * Cm.e[0][j];
-                    v = v + conj(col[1]) * Cm.e[1][j];
-                    v = v + conj(col[2]) * Cm.e[2][j];
-                    S.e[i][j] = S.e[i][j] + v;
-                }
+                for (int j = 0; j < 3; j++)
+                    S.e[i][j] = cjmadd(col[2], Cm.e[2][j], cjmadd(col[1], Cm.e[1][j], cjmadd(col[0], Cm.e[0][j], S.e[i][j])));
             }
         }
     }
@@ -116,16 +101,20 @@ __host__ __device__ __forceinline__ long force_chunks(int Vh, int W) { return 2L
 // mode 0: ipdot = TA(U beta/3 S); mode 1: ipdot += TA(U beta/3 S).
 // One thread per site for one mu: a warp covers 32 consecutive half-sites of one parity, so every
 // link-plane load of the warp is one contiguous 512-byte segment (own links) or nearly so
-// (neighbour links).  mu is the fastest-varying block index, so the four blocks of a site range
-// run together and share their links through L2 (with mu as the slow index the whole link field
-// was streamed from HBM once per mu).  At 3 resident blocks per SM the register budget is 170
-// per thread with no spills.
+// (neighbour links).  The four warps of a block are the four mu of one chunk: of the 76 links they
+// load per site 44 are distinct, and the repeats hit L1 (with mu as the slow index the whole link
+// field was streamed from HBM once per mu).  Bound by FP64 issue (52 %) and L2 latency together:
+// 1,450 FP64 instructions and 19 link loads per link at the 12 warps per SM that 168 registers
+// allow.  32^4: 605 us; 755 us when the products were formed with separate additions (1,900 FP64
+// instructions), 616 us with mu as the fastest block index; 658 us at 16 warps and 128 registers,
+// 700 us at 8 warps.
 __global__ void __launch_bounds__(FORCE_BLOCK, 3) gauge_force_kernel(Geom g, const double2 *__restrict__ U, double *IP,
                                                                       double beta_by_three, int mode)
 {
-    const int mu = blockIdx.x & 3;
+    static_assert(FORCE_BLOCK == 128, "one warp per direction");
+    const int mu = threadIdx.x >> 5;
     const int Vh = g.Vh;
-    const long chunk = (long)(blockIdx.x >> 2) * (FORCE_BLOCK / 32) + (threadIdx.x >> 5);
+    const long chunk = blockIdx.x;
     if (chunk >= force_chunks(Vh, GF_CHUNK)) return;
     const int p = (int)(chunk & 1);
     const int k = (int)(chunk >> 1) * GF_CHUNK + (threadIdx.x & 31);
@@ -203,7 +192,7 @@ __global__ void __launch_bounds__(FORCE_BLOCK, MINB) fermion_force_kernel(Geom g
 
 int gauge_force(rhmc_ctx *c, int mode)
 {
-    const long grid = 4L * grid_for(force_chunks(c->Vh, GF_CHUNK), FORCE_BLOCK / 32);
+    const long grid = force_chunks(c->Vh, GF_CHUNK);
     gauge_force_kernel<<<(unsigned)grid, FORCE_BLOCK, 0, c->stream>>>(c->g, c->U64, c->IP, c->beta / 3.0, mode);
     c->launches++;
     CK(cudaGetLastError());

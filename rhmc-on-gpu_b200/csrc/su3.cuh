@@ -90,6 +90,12 @@ __device__ __forceinline__ void m3_scale(M3 &a, double s)
 
 __device__ __forceinline__ double m3_retr(const M3 &a) { return a.e[0][0].re + a.e[1][1].re + a.e[2][2].re; }
 
+// a b^* + c in four FMAs (a product formed first and then added costs two more operations)
+__device__ __forceinline__ C cmaddc(C a, C b, C c)
+{
+    return mk<double>(c.re + a.re * b.re + a.im * b.im, c.im + a.im * b.re - a.re * b.im);
+}
+
 // link U_mu at (parity p, half index k) of the FP64 master [mu][p][9][Vh] double2
 __device__ __forceinline__ M3 load_link64(const double2 *__restrict__ U, int Vh, int mu, int p, int k)
 {
