@@ -10,9 +10,7 @@
 //   mom_action_kernel   sum 1/2 Tr P^2                (calc_action, action.cc:122-134)
 //   rdot_kernel         Re<a, b> over one parity      (fermion_action, action.cc:65-107)
 //   rational_sum_kernel out = a0 b + sum_i a_i x_i    (rationalapprox.cc:300-311; cuda_sol_sum.cu:168-221)
-// Reductions write per-block FP64 partials that the host sums in block order (deterministic).
-#include <vector>
-
+// Reductions write per-block FP64 partials that one block then sums in a fixed order (deterministic).
 #include "capi_util.h"
 #include "context.h"
 #include "kernels.h"
@@ -66,27 +64,41 @@ __global__ void __launch_bounds__(UPD_BLOCK) link_update_kernel(Geom g, double2 
 }
 
 // temporal and spatial sums of ReTr(U_mu(x) U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag): one thread per
-// site (both parities) and pair of planes, {(0,1),(2,3)}, {(0,2),(1,3)} or {(0,3),(1,2)} (two
-// plaquettes each, every link direction used twice), with the pair as the fastest block index
-// so that the three threads of a site range run together and share its links in L2.
-__global__ void __launch_bounds__(UPD_BLOCK) plaq_kernel(Geom g, const double2 *__restrict__ U, double *partials)
+// site, the six planes in turn.  With X = U_mu(x) U_nu(x+mu) and Y = U_nu(x) U_mu(x+nu) the trace
+// is sum_ij Re(X_ij Y_ij^*): two 3x3 products a plane instead of three.  The site's own links are
+// read for three planes each (L1 hits); warps alternate between the parities, as in force.cu, so
+// that links read as neighbours come from L2.  32^4: 213 us (471 us with three products a plane,
+// formed with separate additions, and three threads a site); 230 us with three threads a site,
+// 238 us at 16 warps per SM; the HBM floor is 93 us, the FP64 floor 87 us.
+constexpr int PLAQ_BLOCK = 128;
+
+__global__ void __launch_bounds__(PLAQ_BLOCK, 3) plaq_kernel(Geom g, const double2 *__restrict__ U, double *partials)
 {
-    const int pair = blockIdx.x % 3;
-    const long t = (long)(blockIdx.x / 3) * blockDim.x + threadIdx.x;
+    const long chunk = (long)blockIdx.x * (PLAQ_BLOCK / 32) + (threadIdx.x >> 5);
     const int Vh = g.Vh;
+    const int p = (int)(chunk & 1), q = 1 - p;
+    const long k0 = (chunk >> 1) * 32 + (threadIdx.x & 31);
     double v[2] = {0.0, 0.0};
-    if (t < 2L * Vh) {
-        const int p = t >= Vh, q = 1 - p;
-        const int k = (int)(t - (long)p * Vh);
+    if (k0 < Vh) {
+        const int k = (int)k0;
         const Site s = site_of(g, p, k);
+#pragma unroll 1
+        for (int pl = 0; pl < 6; pl++) {
+            const int mu = pl < 3 ? 0 : (pl < 5 ? 1 : 2), nu = pl < 3 ? pl + 1 : (pl < 5 ? pl - 1 : 3);
+            const M3 A = load_link64(U, Vh, nu, q, neighbour(g, s, mu, +1));
+            const M3 B = load_link64(U, Vh, mu, q, neighbour(g, s, nu, +1));
+            const M3 M = load_link64(U, Vh, mu, p, k), N = load_link64(U, Vh, nu, p, k);
+            double tr = 0.0;
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int mu = h == 0 ? 0 : (pair == 0 ? 2 : 1);
-            const int nu = h == 0 ? pair + 1 : (pair == 2 ? 2 : 3);
-            M3 a = m3_mul(load_link64(U, Vh, mu, p, k), load_link64(U, Vh, nu, q, neighbour(g, s, mu, +1)));
-            a = m3_mul_nd(a, load_link64(U, Vh, mu, q, neighbour(g, s, nu, +1)));
-            a = m3_mul_nd(a, load_link64(U, Vh, nu, p, k));
-            v[nu == 3 ? 0 : 1] += m3_retr(a);
+            for (int i = 0; i < 3; i++)
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    const C x = cmadd(M.e[i][2], A.e[2][j], cmadd(M.e[i][1], A.e[1][j], M.e[i][0] * A.e[0][j]));
+                    const C y = cmadd(N.e[i][2], B.e[2][j], cmadd(N.e[i][1], B.e[1][j], N.e[i][0] * B.e[0][j]));
+                    tr += x.re * y.re;
+                    tr += x.im * y.im;
+                }
+            v[nu == 3 ? 0 : 1] += tr;
         }
     }
     __shared__ double smem[2 * 32];
@@ -152,14 +164,42 @@ __global__ void __launch_bounds__(UPD_BLOCK) rational_sum_kernel(long nel, int n
     out[i] = make_double2(re, im);
 }
 
-static int host_sum(rhmc_ctx *c, const double *dpart, int nblocks, int n, double *out)
+// out[j] = sum over blocks of part[block][N], in a fixed order: thread t adds blocks t, t + 1024, ...
+constexpr int SUM_BLOCK = 1024;
+
+template <int N>
+__global__ void __launch_bounds__(SUM_BLOCK) sum_partials_kernel(const double *__restrict__ part, int nblocks, double *out)
 {
-    std::vector<double> h((size_t)nblocks * n);
-    CK(cudaMemcpyAsync(h.data(), dpart, h.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    double v[N];
+#pragma unroll
+    for (int j = 0; j < N; j++) v[j] = 0.0;
+#pragma unroll 8
+    for (int b = threadIdx.x; b < nblocks; b += SUM_BLOCK)
+#pragma unroll
+        for (int j = 0; j < N; j++) v[j] += part[(size_t)b * N + j];
+    __shared__ double smem[N * 32];
+    block_sum<N>(v, smem);
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int j = 0; j < N; j++) out[j] = v[j];
+}
+
+// The N sums of nblocks per-block partials, read back through the context's pinned words (behind
+// the solver's polling words).  Summing on the device leaves 8 N bytes to copy; copying every partial
+// to pageable memory and adding them on the host cost 30-60 us per call at 32^4.
+template <int N>
+static int read_sums(rhmc_ctx *c, const double *dpart, int nblocks, double *out)
+{
+    static_assert(N <= 8, "pinned words hold 8 doubles past the polling words");
+    void *tot;
+    CK(c->ws.get("red_tot", 8 * sizeof(double), &tot));
+    sum_partials_kernel<N><<<1, SUM_BLOCK, 0, c->stream>>>(dpart, nblocks, (double *)tot);
+    c->launches++;
+    CK(cudaGetLastError());
+    double *h = reinterpret_cast<double *>(c->hflags) + 8;  // 64 bytes into the 256 pinned ones
+    CK(cudaMemcpyAsync(h, tot, N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    for (int j = 0; j < n; j++) out[j] = 0.0;
-    for (int b = 0; b < nblocks; b++)
-        for (int j = 0; j < n; j++) out[j] += h[(size_t)b * n + j];
+    for (int j = 0; j < N; j++) out[j] = h[j];
     return RHMC_OK;
 }
 
@@ -183,14 +223,14 @@ int link_update(rhmc_ctx *c, double step)
 // sums over all sites of ReTr(plaquette): temporal (nu = 3) and spatial
 int plaquette_sums(rhmc_ctx *c, double *temporal, double *spatial)
 {
-    const int nb = 3 * grid_for(2L * c->Vh, UPD_BLOCK);  // 3 pairs of planes per site range
+    const int nb = grid_for(2L * grid_for(c->Vh, 32), PLAQ_BLOCK / 32);  // a warp per 32 half-sites
     void *part;
     CK(c->ws.get("red_part", (size_t)nb * 2 * sizeof(double), &part));
-    plaq_kernel<<<nb, UPD_BLOCK, 0, c->stream>>>(c->g, c->U64, (double *)part);
+    plaq_kernel<<<nb, PLAQ_BLOCK, 0, c->stream>>>(c->g, c->U64, (double *)part);
     c->launches++;
     CK(cudaGetLastError());
     double o[2] = {0.0, 0.0};
-    int rc = host_sum(c, (const double *)part, nb, 2, o);
+    int rc = read_sums<2>(c, (const double *)part, nb, o);
     *temporal = o[0];
     *spatial = o[1];
     return rc;
@@ -204,7 +244,7 @@ int momentum_action(rhmc_ctx *c, double *out)
     mom_action_kernel<<<nb, UPD_BLOCK, 0, c->stream>>>((int)c->Vh, c->P, (double *)part);
     c->launches++;
     CK(cudaGetLastError());
-    return host_sum(c, (const double *)part, nb, 1, out);
+    return read_sums<1>(c, (const double *)part, nb, out);
 }
 
 int rdot(rhmc_ctx *c, const double2 *a, const double2 *b, long n, double *out)
@@ -215,7 +255,7 @@ int rdot(rhmc_ctx *c, const double2 *a, const double2 *b, long n, double *out)
     rdot_kernel<<<nb, UPD_BLOCK, 0, c->stream>>>(n, a, b, (double *)part);
     c->launches++;
     CK(cudaGetLastError());
-    return host_sum(c, (const double *)part, nb, 1, out);
+    return read_sums<1>(c, (const double *)part, nb, out);
 }
 
 int rational_sum(rhmc_ctx *c, int nrhs, int nshift, double a0, const double *a, const double2 *x, const double2 *b, double2 *out,
