@@ -93,10 +93,6 @@ __global__ void __launch_bounds__(BLOCK, MINB) dslash_kernel(DslashArgs<LF, NR, 
     const int ntiles = (kend - a.k_lo + BLOCK - 1) / BLOCK;
     typedef typename LF::store S;
     typedef typename S::elem E;
-    // y (read only by the epilogue) is fetched into shared memory by cp.async at the start of a
-    // tile, so its DRAM latency overlaps the stencil instead of following it (when it fits)
-    constexpr bool PF = HAS_Y && S::soa && S::pack == 1 && (NR * S::planes * BLOCK * sizeof(E) <= 24576);
-    __shared__ __align__(16) E ysm[PF ? NR * S::planes * BLOCK : 1];
     // tiles of BLOCK consecutive output sites; a launch with fewer blocks than tiles (persistent
     // blocks) walks them with stride gridDim.x, so the per-block work of the fused reduction
     // (fence, ticket) is paid once per block instead of once per tile
@@ -177,15 +173,6 @@ __global__ void __launch_bounds__(BLOCK, MINB) dslash_kernel(DslashArgs<LF, NR, 
             if (RED) reduce_tile<NR>(red, a.partials, tile);
         } else {
             Site s = site_of(a.g, a.p_out, k < kend ? k : a.k_lo);
-            if (PF && k < kend) {
-#pragma unroll
-                for (int r = 0; r < NR; r++)
-#pragma unroll
-                    for (int pl = 0; pl < S::planes; pl++)
-                        cp_async_elem<sizeof(E)>(&ysm[(r * S::planes + pl) * BLOCK + threadIdx.x],
-                                                 a.y + r * a.stride + (size_t)pl * Vh + k);
-                cp_async_commit();
-            }
             double red[NR];
             float tf[NR];
 #pragma unroll
@@ -222,9 +209,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) dslash_kernel(DslashArgs<LF, NR, 
                 for (int r = 0; r < NR; r++) {
                     vec3<R> o;
                     if (HAS_Y) {
-                        if (PF && r == 0) cp_async_wait_all();
-                        const vec3<R> yv = PF ? S::template load_plain<R>(ysm + r * S::planes * BLOCK, BLOCK, threadIdx.x)
-                                              : S::template load<R>(a.y + r * a.stride, Vh, k);
+                        const vec3<R> yv = S::template load<R>(a.y + r * a.stride, Vh, k);
                         const R al = a.use_alphas ? a.alphas[r] : a.alpha;
 #pragma unroll
                         for (int c = 0; c < 3; c++)
@@ -242,10 +227,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) dslash_kernel(DslashArgs<LF, NR, 
                     LF::store::template store<R>(a.out + r * a.stride, Vh, k, o);
                 }
             }
-            if (RED)
-                reduce_tile<NR>(red, a.partials, tile);  // ends with a barrier
-            else if (PF)
-                __syncthreads();  // ysm is refilled by the next tile
+            if (RED) reduce_tile<NR>(red, a.partials, tile);
         }
     }
     if (RED) reduce_last<NR>(a.partials, a.ticket, ntiles * (BLOCK / RED_CHUNK), a.fin);

@@ -14,7 +14,7 @@
 // solver's criterion, cuda_inverter.cu:777-785) or at max_iter.  sigma_0 is the base shift
 // (0 in the reference; the mixed solver uses the smallest pole) and sigma_i are relative to it.
 //
-// Kernel sequence per iteration (one CUDA graph replays a window of MS_WIN iterations):
+// Kernel sequence per iteration (one CUDA graph replays a window of iterations):
 //   K1 D_oe:    h = D_oe p                                   (Dslash, NR right-hand sides)
 //   K2 D_eo:    s = (m^2+sigma_0) p - D_eo h, Re<p,s>        (Dslash epilogue + FP64 reduction;
 //               the last block computes omega, zeta''', omega_i for every RHS)
@@ -32,7 +32,14 @@ namespace rhmc {
 
 constexpr int MS_MAX_SHIFT = 32;
 constexpr int MS_MAX_RHS = 8;
-constexpr int MS_WIN = 8;  // iterations per delayed-update window (= iterations per graph replay)
+// Iterations per delayed-update window (= iterations per graph replay).  A window reads and writes
+// every active shifted vector once (192 bytes per site and system) and costs a ring of MS_WIN
+// residuals per right-hand side and two FP64 coefficients per iteration and system.  With 16 poles
+// and 4 right-hand sides a solve takes 64.5 ms at 24^3x32 (FP64) and 172 ms at 32^4 (FP32 schedule)
+// with 16 iterations per window, 68.8 and 182.7 ms with 8; 32 would not fit the flush's registers.
+// A phase runs windows of MS_WIN or, where the larger ring would not leave the rest of a solve its
+// memory, MS_WIN / 2 iterations (ms_window); the kernels take the length as `win`.
+constexpr int MS_WIN = 16;
 constexpr int VEC_BLOCK = 256;
 
 struct MSRhs {
@@ -60,6 +67,9 @@ struct MSState {
     int stop;     // every RHS finished: K1-K3 skip
     int stop_k4;  // set by the first skipped K1 so that K4 skips from the next iteration on
     int wpos;     // iterations done in the current window (the residual of iteration m is in ring slot m-1)
+    int first;    // no window flushed yet: x_i = 0 and p_i = b are not in memory
+    const double2 *b;  // the right-hand sides (read by the first flush; not a captured argument, so
+                       // that a new b replays the same graph)
     int status;   // 0 ok, 1 iteration cap, 2 non-finite reduction
     int nshift, nrhs, max_iter;
     int stop_on_frozen;             // also stop when every shift is frozen
@@ -84,93 +94,124 @@ constexpr double MS_TAU_REACH = 1e7;
 // FP64 part
 constexpr double MS_TAU_MIN = 1e-4;
 
+// The scalar steps run in every thread of the reduction's last block, thread r the scalars of
+// right-hand side r and one thread per (rhs, shift) the shifted recurrences.  They sit between two
+// launches of the solver, so what counts is their chain of dependent L2 accesses: every thread
+// loads all it needs before the first barrier, and the values of a right-hand side that the
+// (rhs, shift) threads need travel through shared memory.  With thread 0 stepping the right-hand
+// sides one after the other (and counting active shifts one by one) FinAlpha and FinLambda took
+// 5 us each for one right-hand side with 8 shifts and 8 us for four with 16; now 2 us.
+template <int NR>
 struct FinInit {
     MSState *st;
+    int win;
     __device__ void operator()(const double *tot) const
     {
-        if (threadIdx.x != 0) return;
-        for (int r = 0; r < st->nrhs; r++) {
-            MSRhs &q = st->rhs[r];
-            q.b2 = tot[r];
-            q.delta = tot[r];
+        __shared__ int s_any;
+        if (threadIdx.x == 0) s_any = 0;
+        __syncthreads();
+        const int ns = st->nshift;
+        if (threadIdx.x < NR) {
+            MSRhs &q = st->rhs[threadIdx.x];
+            const double b2 = tot[threadIdx.x], res = st->res, tau = st->tau;
+            q.b2 = b2;
+            q.delta = b2;
             q.omega = 1.0;
             q.omega_prev = 1.0;
             q.gamma = 0.0;
-            q.lambda = tot[r];
+            q.lambda = b2;
             q.alpha = 0.0;
             q.iter = 0;
-            q.rslot = MS_WIN - 1;
+            q.rslot = win - 1;
             // precision schedule: the FP64 part ends at tau |b| (tau > 0), or with tau < 0 at
             // -tau |b| but no more than MS_TAU_REACH above the final target
-            const double nb = sqrt(tot[r]);
-            q.res = st->tau > 0.0   ? fmax(st->res, st->tau * nb)
-                    : st->tau < 0.0 ? fmax(st->res, fmax(MS_TAU_MIN * nb, fmin(-st->tau * nb, MS_TAU_REACH * st->res)))
-                                    : st->res;
+            const double nb = sqrt(b2);
+            q.res = tau > 0.0   ? fmax(res, tau * nb)
+                    : tau < 0.0 ? fmax(res, fmax(MS_TAU_MIN * nb, fmin(-tau * nb, MS_TAU_REACH * res)))
+                                : res;
             q.running = 1;
-            q.running_next = (tot[r] > 0.0) ? 1 : 0;  // b == 0: x = 0 is exact
-            if (!isfinite(tot[r])) {
-                st->status = 2;
-                q.running_next = 0;
-            }
-            for (int i = 0; i < st->nshift; i++) {
-                q.zeta_i[i] = 1.0;
-                q.zeta_ii[i] = 1.0;
-                q.zeta_iii[i] = 1.0;
-                q.omegas[i] = 0.0;
-                q.gammas[i] = 0.0;
-                q.active[i] = 1;
-                q.active_next[i] = 1;
-            }
+            const int go = isfinite(b2) && b2 > 0.0;  // b == 0: x = 0 is exact
+            if (!isfinite(b2)) st->status = 2;
+            q.running_next = go;
+            if (go) atomicOr(&s_any, 1);
         }
-        st->stop = 0;
-        st->stop_k4 = 0;
-        int any = 0;
-        for (int r = 0; r < st->nrhs; r++) any |= st->rhs[r].running_next;
-        if (!any) st->stop = 1;
+        for (int t = threadIdx.x; t < NR * ns; t += blockDim.x) {
+            MSRhs &q = st->rhs[t / ns];
+            const int i = t % ns;
+            q.zeta_i[i] = 1.0;
+            q.zeta_ii[i] = 1.0;
+            q.zeta_iii[i] = 1.0;
+            q.omegas[i] = 0.0;
+            q.gammas[i] = 0.0;
+            q.active[i] = 1;
+            q.active_next[i] = 1;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            st->stop = s_any ? 0 : 1;
+            st->stop_k4 = 0;
+            st->first = 1;
+        }
     }
 };
 
-// FinAlpha and FinLambda run in every thread of the reduction's last block: thread 0 steps the
-// scalars of each right-hand side, then one thread per (rhs, shift) the shifted recurrences
-// (independent divisions in parallel instead of one thread's serial chain).
 template <int NR>
 struct FinAlpha {
     MSState *st;
     __device__ void operator()(const double *tot) const
     {
-        if (threadIdx.x == 0) {
-            for (int r = 0; r < NR; r++) {
-                MSRhs &q = st->rhs[r];
-                q.running = q.running_next;
-                if (!q.running) continue;
-                q.alpha = tot[r];
-                if (!isfinite(q.alpha) || q.alpha == 0.0) {
+        __shared__ double s_om[NR], s_omp[NR], s_ga[NR];
+        __shared__ int s_run[NR];
+        const int ns = st->nshift, wp = st->wpos;
+        if (threadIdx.x < NR) {
+            MSRhs &q = st->rhs[threadIdx.x];
+            const double delta = q.delta, prev = q.omega, alpha = tot[threadIdx.x];
+            int run = q.running_next;
+            s_ga[threadIdx.x] = q.gamma;
+            if (run) {
+                q.alpha = alpha;
+                if (!isfinite(alpha) || alpha == 0.0) {
                     st->status = 2;
                     st->stop = 1;
-                    q.running = 0;
                     q.running_next = 0;
-                    continue;
+                    run = 0;
+                } else {
+                    const double om = -delta / alpha;
+                    q.omega_prev = prev;
+                    q.omega = om;
+                    s_omp[threadIdx.x] = prev;
+                    s_om[threadIdx.x] = om;
                 }
-                q.omega_prev = q.omega;
-                q.omega = -q.delta / q.alpha;
             }
+            q.running = run;
+            s_run[threadIdx.x] = run;
         }
-        __syncthreads();
-        const int ns = st->nshift, wp = st->wpos;
-        for (int t = threadIdx.x; t < NR * ns; t += blockDim.x) {
-            const int r = t / ns, i = t % ns;
+        for (int t0 = 0; t0 < NR * ns; t0 += blockDim.x) {
+            const int t = t0 + threadIdx.x, r = t / ns, i = t % ns;
+            const bool in = t < NR * ns;
+            int an = 0;
+            double zi = 1.0, zii = 1.0, sh = 0.0;
+            if (in) {
+                const MSRhs &q = st->rhs[r];
+                an = q.active_next[i];
+                zi = q.zeta_i[i];
+                zii = q.zeta_ii[i];
+                sh = q.shift[i];
+            }
+            if (t0 == 0) __syncthreads();
+            if (!in) continue;
             MSRhs &q = st->rhs[r];
-            const int act = q.running ? q.active_next[i] : 0;
+            const int run = s_run[r], act = run ? an : 0;
             q.h_act[i][wp] = act;
-            if (!q.running) continue;
+            if (!run) continue;
             q.active[i] = act;
             if (!act) continue;
-            const double zi = q.zeta_i[i], zii = q.zeta_ii[i];
-            const double ziii = (zi * zii * q.omega_prev) /
-                                (q.omega * q.gamma * (zi - zii) + zi * q.omega_prev * (1.0 - q.shift[i] * q.omega));
+            const double om = s_om[r], omp = s_omp[r];
+            const double ziii = (zi * zii * omp) / (om * s_ga[r] * (zi - zii) + zi * omp * (1.0 - sh * om));
             q.zeta_iii[i] = ziii;
-            q.omegas[i] = q.omega * ziii / zii;
-            q.h_om[i][wp] = q.omegas[i];
+            const double oms = om * ziii / zii;
+            q.omegas[i] = oms;
+            q.h_om[i][wp] = oms;
         }
     }
 };
@@ -180,64 +221,82 @@ struct FinLambda {
     MSState *st;
     __device__ void operator()(const double *tot) const
     {
-        if (threadIdx.x == 0) {
-            for (int r = 0; r < NR; r++) {
-                MSRhs &q = st->rhs[r];
-                if (!q.running) continue;
-                q.lambda = tot[r];
-                q.rslot = st->wpos;
-                if (!isfinite(q.lambda)) {
+        __shared__ double s_om[NR], s_ga[NR], s_de[NR];
+        __shared__ int s_run[NR], s_nact[NR], s_any;
+        const int ns = st->nshift, wp = st->wpos;
+        double lambda = 0.0, res = 0.0;
+        int run = 0, iter = 0;
+        if (threadIdx.x < NR) {
+            MSRhs &q = st->rhs[threadIdx.x];
+            const double delta = q.delta;
+            run = q.running;
+            iter = q.iter;
+            res = q.res;
+            s_om[threadIdx.x] = q.omega;
+            s_de[threadIdx.x] = delta;
+            s_nact[threadIdx.x] = 0;
+            if (threadIdx.x == 0) s_any = 0;
+            if (run) {
+                lambda = tot[threadIdx.x];
+                q.lambda = lambda;
+                q.rslot = wp;
+                if (!isfinite(lambda)) {
                     st->status = 2;
                     q.running_next = 0;
-                    continue;
+                    run = 0;
+                } else {
+                    const double ga = lambda / delta;
+                    q.gamma = ga;
+                    s_ga[threadIdx.x] = ga;
                 }
-                q.gamma = q.lambda / q.delta;
             }
+            s_run[threadIdx.x] = run;
+        }
+        for (int t0 = 0; t0 < NR * ns; t0 += blockDim.x) {
+            const int t = t0 + threadIdx.x, r = t / ns, i = t % ns;
+            const bool in = t < NR * ns;
+            int act = 0;
+            double zii = 1.0, ziii = 1.0, oms = 0.0, tgt = 0.0;
+            if (in) {
+                const MSRhs &q = st->rhs[r];
+                act = q.active[i];
+                zii = q.zeta_ii[i];
+                ziii = q.zeta_iii[i];
+                oms = q.omegas[i];
+                tgt = st->tgt[i];
+            }
+            if (t0 == 0) __syncthreads();
+            if (!in || !s_run[r] || !act) continue;
+            MSRhs &q = st->rhs[r];
+            const double gas = s_ga[r] * ziii * oms / (zii * s_om[r]);
+            q.gammas[i] = gas;
+            q.h_ga[i][wp] = gas;
+            q.h_ze[i][wp] = ziii;
+            const double fact = sqrt(s_de[r] * zii * zii);
+            const int an = (fact < tgt) ? 0 : 1;
+            q.active_next[i] = an;
+            q.zeta_i[i] = zii;
+            q.zeta_ii[i] = ziii;
+            if (an) atomicAdd(&s_nact[r], 1);
         }
         __syncthreads();
-        const int ns = st->nshift, wp = st->wpos;
-        for (int t = threadIdx.x; t < NR * ns; t += blockDim.x) {
-            const int r = t / ns, i = t % ns;
-            MSRhs &q = st->rhs[r];
-            if (!q.running || !isfinite(q.lambda) || !q.active[i]) continue;
-            q.gammas[i] = q.gamma * q.zeta_iii[i] * q.omegas[i] / (q.zeta_ii[i] * q.omega);
-            q.h_ga[i][wp] = q.gammas[i];
-            q.h_ze[i][wp] = q.zeta_iii[i];
-            const double fact = sqrt(q.delta * q.zeta_ii[i] * q.zeta_ii[i]);
-            q.active_next[i] = (fact < st->tgt[i]) ? 0 : 1;
-            q.zeta_i[i] = q.zeta_ii[i];
-            q.zeta_ii[i] = q.zeta_iii[i];
-        }
-        __syncthreads();
-        if (threadIdx.x != 0) return;
-        int any = 0;
-        for (int r = 0; r < NR; r++) {
-            MSRhs &q = st->rhs[r];
-            if (!q.running || !isfinite(q.lambda)) continue;
-            int nact = 0;
-            for (int i = 0; i < ns; i++) nact += q.active[i] ? q.active_next[i] : 0;
-            q.delta = q.lambda;
-            q.iter++;
-            int done = (sqrt(q.lambda) <= q.res) || (st->stop_on_frozen && nact == 0);
-            if (!done && q.iter >= st->max_iter) {
+        if (run) {  // threads 0..NR-1
+            MSRhs &q = st->rhs[threadIdx.x];
+            q.delta = lambda;
+            q.iter = ++iter;
+            int done = (sqrt(lambda) <= res) || (st->stop_on_frozen && s_nact[threadIdx.x] == 0);
+            if (!done && iter >= st->max_iter) {
                 done = 1;
-                st->status = (st->status == 0) ? 1 : st->status;
+                if (st->status == 0) st->status = 1;
             }
             q.running_next = !done;
-            any |= q.running_next;
+            if (!done) atomicOr(&s_any, 1);
         }
-        for (int r = NR; r < st->nrhs; r++) any |= st->rhs[r].running_next;
-        if (!any) st->stop = 1;
-        st->wpos++;
-    }
-};
-
-// end of a window (after ms_flush_kernel has read its scalars)
-struct FinWindow {
-    MSState *st;
-    __device__ void operator()(const double *) const
-    {
-        if (threadIdx.x == 0) st->wpos = 0;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            if (!s_any) st->stop = 1;
+            st->wpos = wp + 1;
+        }
     }
 };
 
@@ -267,18 +326,16 @@ __host__ __device__ __forceinline__ size_t bidx(int j, int c, int k, int Vh)
     return ((size_t)((j / P) * 3 + c) * Vh + k) * P + (j % P);
 }
 
-// x_i = 0, r_0 = p = p_i = b (b FP64 internal), |b|^2.  r_0 goes to the last slot of the
-// residual ring (the slot the first iteration reads).  Base vectors (ring, p) are stored in Rv,
-// the shifted solutions and directions (x, ps) in Rx.
-template <typename Rv, typename Rx, int NR>
-__global__ void __launch_bounds__(VEC_BLOCK) ms_init_kernel(int Vh, int nshift, size_t stride, const double2 *__restrict__ b,
+// r_0 = p = b (b FP64 internal), |b|^2.  r_0 goes to the last slot of the residual ring (the slot
+// the first iteration reads).  The shifted x_i = 0 and p_i = b are not written: the first window's
+// flush starts from them without reading any (MSState::first).
+template <typename Rv, int NR>
+__global__ void __launch_bounds__(VEC_BLOCK) ms_init_kernel(int Vh, size_t stride, int win, const double2 *__restrict__ b,
                                                              typename MSVec<Rv>::E *ring, typename MSVec<Rv>::E *p,
-                                                             typename MSVec<Rx>::E *ps, typename MSVec<Rx>::E *x,
                                                              double *partials, unsigned *ticket, MSState *st)
 {
-    typename MSVec<Rv>::E *r = ring + (size_t)(MS_WIN - 1) * NR * stride;
+    typename MSVec<Rv>::E *r = ring + (size_t)(win - 1) * NR * stride;
     typedef typename MSVec<Rv>::E E;
-    typedef typename MSVec<Rx>::E EX;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     double red[NR];
 #pragma unroll
@@ -288,41 +345,31 @@ __global__ void __launch_bounds__(VEC_BLOCK) ms_init_kernel(int Vh, int nshift, 
         for (int j = 0; j < NR; j++) {
 #pragma unroll
             for (int c = 0; c < 3; c++) {
-                const size_t o = j * stride + (size_t)c * Vh + k, ob = bidx<Rv, NR>(j, c, k, Vh);
-                const double2 v = b[o];
+                const size_t ob = bidx<Rv, NR>(j, c, k, Vh);
+                const double2 v = b[j * stride + (size_t)c * Vh + k];
                 red[j] += dot2(v.x, v.x, v.y, v.y);
                 E e;
                 e.x = (Rv)v.x;
                 e.y = (Rv)v.y;
                 r[ob] = e;
                 p[ob] = e;
-                EX ex, z;
-                ex.x = (Rx)v.x;
-                ex.y = (Rx)v.y;
-                z.x = 0;
-                z.y = 0;
-                for (int i = 0; i < nshift; i++) {
-                    const size_t oi = (size_t)(j * nshift + i) * stride + (size_t)c * Vh + k;
-                    ps[oi] = ex;
-                    x[oi] = z;
-                }
             }
         }
     }
-    FinInit fin{st};
+    FinInit<NR> fin{st, win};
     reduce_finalize<NR>(red, partials, ticket, fin);
 }
 
 // r_m = r_{m-1} + omega s (ring slots wpos-1 -> wpos), |r_m|^2 per RHS
 template <typename Rv, int NR>
-__global__ void __launch_bounds__(VEC_BLOCK) ms_resid_kernel(int Vh, size_t stride, typename MSVec<Rv>::E *ring,
+__global__ void __launch_bounds__(VEC_BLOCK) ms_resid_kernel(int Vh, size_t stride, int win, typename MSVec<Rv>::E *ring,
                                                               const typename MSVec<Rv>::E *__restrict__ s, double *partials,
                                                               unsigned *ticket, MSState *st)
 {
     typedef typename MSVec<Rv>::E E;
     if (*(volatile int *)&st->stop) return;
     const int wp = *(volatile const int *)&st->wpos;
-    const E *rprev = ring + (size_t)((wp + MS_WIN - 1) % MS_WIN) * NR * stride;
+    const E *rprev = ring + (size_t)(wp == 0 ? win - 1 : wp - 1) * NR * stride;
     E *r = ring + (size_t)wp * NR * stride;
     int run[NR];
     Rv om[NR];
@@ -393,7 +440,7 @@ __global__ void __launch_bounds__(VEC_BLOCK) ms_update_kernel(int Vh, size_t str
     if (*(volatile int *)&st->stop_k4) return;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= Vh) return;
-    const E *r = ring + (size_t)((*(volatile const int *)&st->wpos + MS_WIN - 1) % MS_WIN) * NR * stride;
+    const E *r = ring + (size_t)(*(volatile const int *)&st->wpos - 1) * NR * stride;  // K3 advanced wpos
 #pragma unroll
     for (int q = 0; q < NR / P; q++) {
         int run[P], any = 0;
@@ -422,106 +469,140 @@ __global__ void __launch_bounds__(VEC_BLOCK) ms_update_kernel(int Vh, size_t str
     }
 }
 
-// End of a window of m = wpos iterations with residuals r_1..r_m (ring slots 0..m-1).  Over the
-// window the per-iteration updates x_i -= om_k p_i, p_i = ze_k r_k + ga_k p_i compose to
-//   x_i = X0_i - cx0 P0_i - sum_k cx_k r_k,   p_i = ca P0_i + sum_k cb_k r_k
-// with P0_i, X0_i the stored vectors of the window start.  The first NR*nshift threads of every
-// block derive (cx0, cx, ca, cb) of one (rhs, shift) from the recorded scalars into shared memory
-// (skipping iterations where the shift was frozen), then every site applies them: each shifted
-// vector is read and written once per window instead of once per iteration.
-template <typename Rv, typename Rx, int NR>
-__global__ void __launch_bounds__(VEC_BLOCK) ms_flush_kernel(int Vh, int nshift, size_t stride,
-                                                              const typename MSVec<Rv>::E *__restrict__ ring,
-                                                              typename MSVec<Rx>::E *ps, typename MSVec<Rx>::E *x,
-                                                              double *partials, unsigned *ticket, MSState *st)
+// End of a window of wpos iterations with residuals r_0..r_{wpos-1} (ring slots).  Over the window
+// the per-iteration updates x_i -= om_m p_i, p_i = ze_m r_m + ga_m p_i compose to
+//   x_i = X0_i - cx0 P0_i - sum_m cx_m r_m,   p_i = ca P0_i + sum_m cb_m r_m
+// with P0_i, X0_i the vectors at the window start (b and 0 in the first window).  Backwards over
+// the window, with D the coefficient of the direction entering iteration m+1 in x and G that in p,
+//   cx_m = ze_m D, cb_m = ze_m G, D <- om_m + ga_m D, G <- ga_m G   (frozen iterations skipped)
+// and cx0 = D, ca = G at the end.  Warp j of every block derives the coefficients of right-hand
+// side j (lane i: shift i) into shared memory and lists its active shifts; then a thread per site
+// and right-hand side of a pack (the pack index fastest, so the lanes of a warp read whole packs)
+// holds the window's residuals of one colour in registers and streams every active x_i, p_i
+// through, the next one's loads issued before the current one's arithmetic.
+template <typename Rv, int NR>
+__global__ void __launch_bounds__(VEC_BLOCK, 2) ms_flush_kernel(int Vh, int nshift, size_t stride,
+                                                                 const typename MSVec<Rv>::E *__restrict__ ring, double2 *ps,
+                                                                 double2 *x, unsigned *ticket, MSState *st)
 {
-    typedef typename MSVec<Rx>::E E;
-    __shared__ double s_cx0[NR * MS_MAX_SHIFT], s_ca[NR * MS_MAX_SHIFT];
-    __shared__ double s_cx[NR * MS_MAX_SHIFT][MS_WIN], s_cb[NR * MS_MAX_SHIFT][MS_WIN];
-    __shared__ int s_use[NR * MS_MAX_SHIFT];  // 0: nothing to do, 1: x only, 2: x and p
-    const int wp = *(volatile const int *)&st->wpos;
-    for (int t = threadIdx.x; t < NR * nshift; t += blockDim.x) {
-        const int j = t / nshift, i = t % nshift;
-        const MSRhs &q = st->rhs[j];
-        double cx0 = 0.0, ca = 1.0, cx[MS_WIN], cb[MS_WIN];
-        int any = 0;
-        for (int m = 0; m < MS_WIN; m++) cx[m] = cb[m] = 0.0;
-        for (int m = 0; m < wp; m++) {
-            if (!q.h_act[i][m]) continue;
-            any = 1;
-            const double om = q.h_om[i][m], ga = q.h_ga[i][m];
-            cx0 += om * ca;
-            for (int l = 0; l < m; l++) cx[l] += om * cb[l];
-            ca *= ga;
-            for (int l = 0; l < m; l++) cb[l] *= ga;
-            cb[m] = q.h_ze[i][m];
+    extern __shared__ double2 s_coef[];  // [rhs][nshift][MS_WIN + 1] (cx, cb), entry MS_WIN (cx0, ca)
+    __shared__ int s_list[NR][MS_MAX_SHIFT], s_n[NR];  // active shifts, 2 i + (p_i is needed further)
+    static_assert(NR <= VEC_BLOCK / 32 && MS_MAX_SHIFT <= 32, "a warp per right-hand side, a lane per shift");
+    constexpr int P = BasePack<Rv, NR>::P;
+    const int rstride = nshift * (MS_WIN + 1) + 1;  // one element of padding: other banks for another RHS
+    const int wp = *(volatile const int *)&st->wpos, first = *(volatile const int *)&st->first;
+    {
+        const int j = threadIdx.x >> 5, i = threadIdx.x & 31;
+        if (j < NR) {
+            int any = 0, an = 0;
+            if (i < nshift) {
+                const MSRhs &q = st->rhs[j];
+                double2 *cf = s_coef + (size_t)j * rstride + i * (MS_WIN + 1);
+                an = q.active_next[i];
+                double D = 0.0, G = 1.0;
+                // the window's scalars loaded in batches (entries past wp or of frozen iterations are
+                // stale and not used): one L2 latency per batch instead of one per iteration
+                constexpr int B = 8;
+                static_assert(MS_WIN % B == 0, "whole batches");
+#pragma unroll
+                for (int m0 = MS_WIN - B; m0 >= 0; m0 -= B) {
+                    double om[B], ga[B], ze[B];
+                    int act[B];
+#pragma unroll
+                    for (int m = 0; m < B; m++) {
+                        om[m] = q.h_om[i][m0 + m];
+                        ga[m] = q.h_ga[i][m0 + m];
+                        ze[m] = q.h_ze[i][m0 + m];
+                        act[m] = m0 + m < wp ? q.h_act[i][m0 + m] : 0;
+                    }
+#pragma unroll
+                    for (int m = B - 1; m >= 0; m--) {
+                        cf[m0 + m] = act[m] ? make_double2(ze[m] * D, ze[m] * G) : make_double2(0.0, 0.0);
+                        if (act[m]) {
+                            D = om[m] + ga[m] * D;
+                            G = ga[m] * G;
+                            any = 1;
+                        }
+                    }
+                }
+                cf[MS_WIN] = make_double2(D, G);
+            }
+            // p_i is written for every shift still active, also when the RHS stopped in this window:
+            // a later phase may resume it from exactly this state.  The first window visits every
+            // shift: x_i is in memory only after it.
+            const int use = i < nshift && (any || first);
+            const unsigned mask = __ballot_sync(0xffffffffu, use);
+            if (use) s_list[j][__popc(mask & ((1u << i) - 1u))] = 2 * i + (an ? 1 : 0);
+            if (i == 0) s_n[j] = __popc(mask);
         }
-        s_cx0[t] = cx0;
-        s_ca[t] = ca;
-        for (int m = 0; m < MS_WIN; m++) {
-            s_cx[t][m] = cx[m];
-            s_cb[t][m] = cb[m];
-        }
-        // p_i is written for every shift still active, also when the RHS stopped in this window:
-        // a later phase may resume it from exactly this state
-        s_use[t] = any ? (q.active_next[i] ? 2 : 1) : 0;
     }
     __syncthreads();
-    constexpr int P = BasePack<Rv, NR>::P;
-    typedef PackIO<Rv, P> IO;
-    typedef PackElem<Rv, P> PE;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < Vh && wp > 0) {
+    const long id = (long)blockIdx.x * VEC_BLOCK + threadIdx.x;
+    const int k = (int)(id / P), l = (int)(id % P);
+    if (k < Vh && (wp > 0 || first)) {
         for (int q = 0; q < NR / P; q++) {
-#pragma unroll
+            const int j = q * P + l, n = s_n[j];
+            if (n == 0) continue;
+            const double2 *cj = s_coef + (size_t)j * rstride;
+#pragma unroll 1
             for (int c = 0; c < 3; c++) {
-                // the window's residuals of this site, read once (a pack of P right-hand sides per
-                // load) and shared by every shift
-                cpx<Rv> rp[MS_WIN][P];
+                const size_t o = (size_t)j * nshift * stride + (size_t)c * Vh + k;
+                double2 rv[MS_WIN];  // slots past wp hold older residuals and have zero coefficients
 #pragma unroll
-                for (int m = 0; m < MS_WIN; m++)
-                    if (m < wp) IO::ld((const PE *)(ring + (size_t)m * NR * stride) + bidx<Rv, NR>(q * P, c, k, Vh) / P, rp[m]);
-#pragma unroll
-                for (int l = 0; l < P; l++) {
-                    const int j = q * P + l;
-                    E rv[MS_WIN];
-#pragma unroll
-                    for (int m = 0; m < MS_WIN; m++)
-                        if (m < wp) {
-                            rv[m].x = (Rx)rp[m][l].re;
-                            rv[m].y = (Rx)rp[m][l].im;
-                        }
-                    for (int i = 0; i < nshift; i++) {
-                        const int t = j * nshift + i, use = s_use[t];
-                        if (!use) continue;
-                        const size_t o = (size_t)t * stride + (size_t)c * Vh + k;
-                        const Rx x0 = (Rx)s_cx0[t], a0 = (Rx)s_ca[t];
-                        const E p0 = ps[o];
-                        E xv = x[o];
-                        E pv;
-                        xv.x = xv.x - x0 * p0.x;
-                        xv.y = xv.y - x0 * p0.y;
-                        pv.x = a0 * p0.x;
-                        pv.y = a0 * p0.y;
-#pragma unroll
-                        for (int m = 0; m < MS_WIN; m++) {
-                            if (m >= wp) break;
-                            const Rx cx = (Rx)s_cx[t][m], cb = (Rx)s_cb[t][m];
-                            xv.x = xv.x - cx * rv[m].x;
-                            xv.y = xv.y - cx * rv[m].y;
-                            pv.x = pv.x + cb * rv[m].x;
-                            pv.y = pv.y + cb * rv[m].y;
-                        }
-                        x[o] = xv;
-                        if (use == 2) ps[o] = pv;
+                for (int m = 0; m < MS_WIN; m++) {
+                    rv[m] = make_double2(0.0, 0.0);
+                    if (m < wp) {
+                        const typename MSVec<Rv>::E e = __ldg(ring + (size_t)m * NR * stride + bidx<Rv, NR>(j, c, k, Vh));
+                        rv[m] = make_double2((double)e.x, (double)e.y);
                     }
+                }
+                double2 pn, xn = make_double2(0.0, 0.0);
+                int en = s_list[j][0];
+                if (first) {
+                    pn = __ldg(st->b + (size_t)j * stride + (size_t)c * Vh + k);
+                } else {
+                    pn = ps[o + (size_t)(en >> 1) * stride];
+                    xn = x[o + (size_t)(en >> 1) * stride];
+                }
+                for (int t = 0; t < n; t++) {
+                    const int e = en, i = e >> 1;
+                    const double2 p0 = pn;
+                    double2 xv = xn;
+                    if (t + 1 < n) {
+                        en = s_list[j][t + 1];
+                        if (!first) {
+                            pn = ps[o + (size_t)(en >> 1) * stride];
+                            xn = x[o + (size_t)(en >> 1) * stride];
+                        }
+                    }
+                    const double2 *cf = cj + i * (MS_WIN + 1);
+                    const double2 c0 = cf[MS_WIN];
+                    double2 pv;
+                    xv.x = xv.x - c0.x * p0.x;
+                    xv.y = xv.y - c0.x * p0.y;
+                    pv.x = c0.y * p0.x;
+                    pv.y = c0.y * p0.y;
+#pragma unroll
+                    for (int m = 0; m < MS_WIN; m++) {
+                        const double2 cm = cf[m];
+                        xv.x = xv.x - cm.x * rv[m].x;
+                        xv.y = xv.y - cm.x * rv[m].y;
+                        pv.x = pv.x + cm.y * rv[m].x;
+                        pv.y = pv.y + cm.y * rv[m].y;
+                    }
+                    x[o + (size_t)i * stride] = xv;
+                    if (e & 1) ps[o + (size_t)i * stride] = pv;
                 }
             }
         }
     }
-    double none[1] = {0.0};
-    FinWindow fin{st};
-    reduce_finalize<1>(none, partials, ticket, fin);
+    // the last block to get here starts a new window; every thread of a block read wpos and first
+    // before the barrier above, so the reset cannot reach one that still needs them
+    if (threadIdx.x == 0 && atomicAdd(ticket, 1u) == gridDim.x - 1) {
+        *ticket = 0;
+        st->wpos = 0;
+        st->first = 0;
+    }
 }
 
 // ------------------------------------------------------------------ precision-scheduled resumption
@@ -561,7 +642,7 @@ static __global__ void ms_rearm_kernel(MSState *st)
 template <typename Rf, typename Rt, int NR>
 __global__ void __launch_bounds__(VEC_BLOCK) ms_convert_kernel(int Vh, size_t stride, const typename MSVec<Rf>::E *__restrict__ ring_f,
                                                                 const typename MSVec<Rf>::E *__restrict__ p_f,
-                                                                typename MSVec<Rt>::E *ring_t, typename MSVec<Rt>::E *p_t,
+                                                                typename MSVec<Rt>::E *ring_t, typename MSVec<Rt>::E *p_t, int win,
                                                                 const MSState *st)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -578,7 +659,7 @@ __global__ void __launch_bounds__(VEC_BLOCK) ms_convert_kernel(int Vh, size_t st
             a.y = (Rt)rv.y;
             b.x = (Rt)pv.x;
             b.y = (Rt)pv.y;
-            ring_t[(size_t)(MS_WIN - 1) * NR * stride + ot] = a;
+            ring_t[(size_t)(win - 1) * NR * stride + ot] = a;
             p_t[ot] = b;
         }
     }
@@ -654,7 +735,7 @@ struct FinMsRU {
 // base direction is re-synchronised with the FP64 shifted direction of the base shift (both
 // follow the same recurrence; the sloppy copy drifts by rounding).  |r|^2 becomes delta.
 template <typename Rv, int NR>
-__global__ void __launch_bounds__(VEC_BLOCK) ms_ru_resid_kernel(int Vh, int nshift, size_t stride, const double2 *__restrict__ b,
+__global__ void __launch_bounds__(VEC_BLOCK) ms_ru_resid_kernel(int Vh, int nshift, size_t stride, int win, const double2 *__restrict__ b,
                                                                  const double2 *__restrict__ t, const double2 *__restrict__ ps,
                                                                  typename MSVec<Rv>::E *ring, typename MSVec<Rv>::E *p,
                                                                  double *partials, unsigned *ticket, MSState *st)
@@ -681,7 +762,7 @@ __global__ void __launch_bounds__(VEC_BLOCK) ms_ru_resid_kernel(int Vh, int nshi
                 e.y = (Rv)im;
                 f.x = (Rv)pv.x;
                 f.y = (Rv)pv.y;
-                ring[(size_t)(MS_WIN - 1) * NR * stride + ob] = e;
+                ring[(size_t)(win - 1) * NR * stride + ob] = e;
                 p[ob] = f;
             }
         }

@@ -35,8 +35,8 @@
 namespace rhmc {
 
 constexpr int RB_MAX = 8;
-// windows (of MS_WIN iterations) between reliable updates of the FP32 multi-shift phase
-constexpr int MX_RU_WINDOWS = 4;
+// iterations between reliable updates of the FP32 multi-shift phase
+constexpr int MX_RU_ITERS = 32;
 
 // one translation unit per link format (refine_run.cuh, inst_*.cu)
 template <class LF>
@@ -132,7 +132,7 @@ int msolve_mixed(rhmc_ctx *c, int fmt, int nshift, const double *shifts, int nrh
     } else {
         // Precision schedule: FP64 (12-real links) until |r| <= tol_A |b| for every RHS, then the
         // same recurrences resumed with FP32 links and base vectors, FP64 shifted vectors and a
-        // reliable update of the base system every MX_RU_WINDOWS windows, to the final target.
+        // reliable update of the base system every MX_RU_ITERS iterations, to the final target.
         for (double &t : tgt) t = res;
         A.tgt = tgt.data();
         A.res_base = res;
@@ -144,7 +144,7 @@ int msolve_mixed(rhmc_ctx *c, int fmt, int nshift, const double *shifts, int nrh
         if (rc == RHMC_OK) {
             A.fresh = 0;
             A.tau = 0.0;
-            A.ru_every = MX_RU_WINDOWS;
+            A.ru_every = MX_RU_ITERS;
             // half refinement follows an FP32 multi-shift on 12-real links
             rc = msolve_shifted(c, fmt == RHMC_LINKS_F16_12 ? RHMC_LINKS_F32_12 : fmt, A, &mi);
             if (rc && rc != RHMC_ERR_MAXITER) return rc;

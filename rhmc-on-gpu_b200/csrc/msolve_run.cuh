@@ -19,6 +19,19 @@ static inline int vec_grid(rhmc_ctx *c) { return grid_for(c->Vh, VEC_BLOCK); }
 // workspace slot name of a base vector set in elements of `bytes` bytes
 static inline std::string vname(const char *base, size_t bytes) { return std::string(base) + std::to_string(bytes); }
 
+// Iterations per window of a phase whose residual ring takes `slot` bytes per iteration: MS_WIN when
+// the ring is already that long or fits with room to spare for what the rest of a solve may still
+// allocate (true residuals 16, refinement at most 52 FP64 spinors of v64 bytes), else half of it.
+static inline int ms_window(rhmc_ctx *c, const std::string &name, size_t slot, size_t v64)
+{
+    const auto it = c->ws.buf.find(name);
+    const size_t have = it == c->ws.buf.end() ? 0 : it->second.second;
+    if (have >= MS_WIN * slot) return MS_WIN;
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) return MS_WIN / 2;
+    return free_bytes + have >= MS_WIN * slot + 68 * v64 ? MS_WIN : MS_WIN / 2;
+}
+
 // One phase of the multi-shift CG with links LF: base vectors (residual ring, p, h, s) in the
 // links' precision, shifted solutions and directions always FP64.  A fresh phase starts from
 // x_i = 0; a resumed phase continues the state a previous FP64 phase left (scalars, shifted
@@ -37,7 +50,6 @@ static int ms_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *
     const bool ru = A.ru_every > 0;
     if (!A.fresh && sizeof(E) == sizeof(double2)) return fail(RHMC_ERR_ARG, "multi-shift: an FP64 phase cannot resume an FP64 phase");
     void *r, *p, *h, *s, *ps, *stv, *part, *tick;
-    CK(c->ws.get(vname("ms_r", sizeof(E)), (size_t)MS_WIN * NR * vbytes, &r));  // ring of the window's residuals [slot][rhs]
     CK(c->ws.get(vname("ms_p", sizeof(E)), NR * vbytes, &p));
     CK(c->ws.get(vname("ms_h", sizeof(E)), NR * vbytes, &h));
     CK(c->ws.get(vname("ms_s", sizeof(E)), NR * vbytes, &s));
@@ -46,6 +58,10 @@ static int ms_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *
     const int gv = vec_grid(c);
     CK(c->ws.get("ms_partials", (size_t)red_chunks(Vh) * 2 * NR * sizeof(double), &part));
     CK(c->ws.get("ms_tickets", 8 * sizeof(unsigned), &tick));
+    // ring of the window's residuals [slot][rhs]
+    const int win = ms_window(c, vname("ms_r", sizeof(E)), NR * vbytes, v64);
+    CK(c->ws.get(vname("ms_r", sizeof(E)), (size_t)win * NR * vbytes, &r));
+    const int ru_every = (A.ru_every + win - 1) / win;  // in windows
     MSState *st = (MSState *)stv;
     unsigned *tk = (unsigned *)tick;
     double *pt = (double *)part;
@@ -60,7 +76,7 @@ static int ms_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *
         h0.stop_on_frozen = A.stop_on_frozen;
         h0.res = A.res_base;
         h0.tau = A.tau;
-        h0.ru_every = A.ru_every;
+        h0.ru_every = ru_every;
         for (int i = 0; i < S; i++) h0.tgt[i] = A.tgt[i];
         for (int rr = 0; rr < NR; rr++) {
             int i0 = -1;  // the pole the RHS iterates on (reliable updates need it among the poles)
@@ -72,22 +88,22 @@ static int ms_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *
             h0.rhs[rr].i0 = i0 < 0 ? 0 : i0;
         }
         h0.wpos = 0;
+        h0.b = (const double2 *)A.b;
         CK(cudaMemcpyAsync(st, &h0, sizeof(MSState), cudaMemcpyHostToDevice, s_));
         CK(cudaMemsetAsync(tk, 0, 8 * sizeof(unsigned), s_));
-        ms_init_kernel<Rv, double, NR><<<gv, VEC_BLOCK, 0, s_>>>(Vh, S, stride, (const double2 *)A.b, (E *)r, (E *)p,
-                                                                 (double2 *)ps, xs, pt, tk, st);
+        ms_init_kernel<Rv, NR><<<gv, VEC_BLOCK, 0, s_>>>(Vh, stride, win, (const double2 *)A.b, (E *)r, (E *)p, pt, tk, st);
         c->launches++;
         CK(cudaGetLastError());
     } else {
-        // resume the FP64 phase's state in this phase's precision
+        // resume the FP64 phase's state in this phase's precision (its ring as long as that phase made it)
         void *r64, *p64;
-        CK(c->ws.get(vname("ms_r", sizeof(double2)), (size_t)MS_WIN * NR * v64, &r64));
+        CK(c->ws.get(vname("ms_r", sizeof(double2)), NR * v64, &r64));
         CK(c->ws.get(vname("ms_p", sizeof(double2)), NR * v64, &p64));
         CK(cudaMemcpyAsync(&st->res, &A.res_base, sizeof(double), cudaMemcpyHostToDevice, s_));
-        CK(cudaMemcpyAsync(&st->ru_every, &A.ru_every, sizeof(int), cudaMemcpyHostToDevice, s_));
+        CK(cudaMemcpyAsync(&st->ru_every, &ru_every, sizeof(int), cudaMemcpyHostToDevice, s_));
         ms_rearm_kernel<<<1, 32, 0, s_>>>(st);
         ms_convert_kernel<double, Rv, NR><<<gv, VEC_BLOCK, 0, s_>>>(Vh, stride, (const double2 *)r64, (const double2 *)p64,
-                                                                     (E *)r, (E *)p, st);
+                                                                     (E *)r, (E *)p, win, st);
         c->launches += 2;
         CK(cudaGetLastError());
     }
@@ -147,7 +163,11 @@ static int ms_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *
         for (int rr = 0; rr < NR; rr++) u2.alphas[rr] = c->mass * c->mass + A.base[rr];
     }
 
-    const int chunk = MS_WIN;  // one graph replay = one delayed-update window
+    // shared memory of the flush's coefficients: above the 48 KB default for wide batches of many poles
+    const size_t coef_bytes = (size_t)NR * (S * (MS_WIN + 1) + 1) * sizeof(double2);
+    if (coef_bytes > 48 * 1024)
+        CK(cudaFuncSetAttribute(ms_flush_kernel<Rv, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)coef_bytes));
+    const int chunk = win;  // one graph replay = one delayed-update window
     struct Key {
         int kind, link_reals, link_bytes, nr, chunk, nshift, vh, ru_every;
         const void *links, *links64, *r, *p, *h, *s, *ps, *xs, *pt, *tk, *st, *x0, *h64, *t64, *b;
@@ -164,7 +184,7 @@ static int ms_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *
         key.cand[3] = dslash_candidate<L64_12, NR, true, false>(c->g, l64, s_);
     }
     key.kind = 4; key.link_reals = LF::reals; key.link_bytes = (int)sizeof(typename LF::real); key.nr = NR;
-    key.chunk = chunk; key.nshift = S; key.vh = Vh; key.ru_every = A.ru_every; key.links = lf.p; key.r = r; key.p = p;
+    key.chunk = chunk; key.nshift = S; key.vh = Vh; key.ru_every = ru_every; key.links = lf.p; key.r = r; key.p = p;
     key.h = h; key.s = s; key.ps = ps; key.xs = xs; key.pt = pt; key.tk = tk; key.st = st; key.stream = s_;
     if (ru) {
         key.links64 = l64.p; key.x0 = x0; key.h64 = h64; key.t64 = t64; key.b = A.b;
@@ -180,16 +200,17 @@ static int ms_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *
             dslash_launch_cand<LFB, NR, false, false, NoFin>(key.cand[0], a1, Vh, s_);
             dslash_launch_cand<LFB, NR, true, true, FinAlpha<NR>>(key.cand[1], a2, Vh, s_);
             ms_resid_kernel<Rv, NR><<<persistent_grid((const void *)ms_resid_kernel<Rv, NR>, VEC_BLOCK, gv), VEC_BLOCK, 0,
-                                      s_>>>(Vh, stride, (E *)r, (const E *)s, pt, tk + 2, st);
+                                      s_>>>(Vh, stride, win, (E *)r, (const E *)s, pt, tk + 2, st);
             ms_update_kernel<Rv, NR><<<gv, VEC_BLOCK, 0, s_>>>(Vh, stride, (const E *)r, (E *)p, st);
         }
-        ms_flush_kernel<Rv, double, NR><<<gv, VEC_BLOCK, 0, s_>>>(Vh, S, stride, (const E *)r, (double2 *)ps, xs, pt, tk + 3, st);
+        ms_flush_kernel<Rv, NR><<<grid_for((long)Vh * BasePack<Rv, NR>::P, VEC_BLOCK), VEC_BLOCK, coef_bytes, s_>>>(
+            Vh, S, stride, (const E *)r, (double2 *)ps, xs, tk + 3, st);
         if (ru) {
             ms_ru_begin_kernel<<<1, 32, 0, s_>>>(st);
             ms_gather_base_kernel<NR><<<gv, VEC_BLOCK, 0, s_>>>(Vh, S, stride, xs, (double2 *)x0, st);
             dslash_launch_cand<L64_12, NR, false, false, NoFin>(key.cand[2], u1, Vh, s_);
             dslash_launch_cand<L64_12, NR, true, false, NoFin>(key.cand[3], u2, Vh, s_);
-            ms_ru_resid_kernel<Rv, NR><<<gv, VEC_BLOCK, 0, s_>>>(Vh, S, stride, (const double2 *)A.b, (const double2 *)t64,
+            ms_ru_resid_kernel<Rv, NR><<<gv, VEC_BLOCK, 0, s_>>>(Vh, S, stride, win, (const double2 *)A.b, (const double2 *)t64,
                                                                   (const double2 *)ps, (E *)r, (E *)p, pt, tk + 4, st);
         }
         ce = cudaStreamEndCapture(s_, &graph);

@@ -348,7 +348,6 @@ struct F64S {
         for (int c = 0; c < 3; c++) d.c[c] = mk<double>((double)r.c[c].re, (double)r.c[c].im);
         store_spinor<double>(v, Vh, k, d);
     }
-    // the same from memory that __ldg cannot address (shared), planes pstride elements apart
     template <typename R>
     __device__ __forceinline__ static vec3<R> load_plain(const elem *v, int pstride, int k)
     {
@@ -459,11 +458,6 @@ struct H16S {
         return decode<R>(__ldg(v + k));
     }
     template <typename R>
-    __device__ __forceinline__ static vec3<R> load_plain(const elem *v, int, int k)
-    {
-        return decode<R>(v[k]);
-    }
-    template <typename R>
     __device__ __forceinline__ static vec3<R> decode(const uint4 q)
     {
         const float nrm = __uint_as_float(q.w);
@@ -492,21 +486,6 @@ struct H16S {
         v[k] = q;
     }
 };
-
-// asynchronous global -> shared copy of one element (cp.async: no registers held while in flight)
-template <int BYTES>
-__device__ __forceinline__ void cp_async_elem(void *smem, const void *gmem)
-{
-    static_assert(BYTES == 4 || BYTES == 8 || BYTES == 16, "cp.async copies 4, 8 or 16 bytes");
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    const size_t ga = __cvta_generic_to_global(gmem);
-    if constexpr (BYTES == 16)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(ga) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(sa), "l"(ga), "n"(BYTES) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // ------------------------------------------------------------------ packed right-hand sides
 // A batch of right-hand sides stored P at a time: element (pack q, colour c, site k) holds the P
