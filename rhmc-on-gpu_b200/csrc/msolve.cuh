@@ -26,6 +26,8 @@
 // Scalars live in device memory (MSState) and never leave the GPU during the solve; the host
 // only polls the stop flag between graph replays.
 #pragma once
+#include <cstddef>
+
 #include "dslash.cuh"
 
 namespace rhmc {
@@ -38,7 +40,7 @@ constexpr int MS_MAX_RHS = 8;
 // and 4 right-hand sides a solve takes 64.5 ms at 24^3x32 (FP64) and 172 ms at 32^4 (FP32 schedule)
 // with 16 iterations per window, 68.8 and 182.7 ms with 8; 32 would not fit the flush's registers.
 // A phase runs windows of MS_WIN or, where the larger ring would not leave the rest of a solve its
-// memory, MS_WIN / 2 iterations (ms_window); the kernels take the length as `win`.
+// memory, MS_WIN / 2 iterations (ms_ring); the kernels take the length as `win`.
 constexpr int MS_WIN = 16;
 constexpr int VEC_BLOCK = 256;
 
@@ -57,10 +59,13 @@ struct MSRhs {
     int active[MS_MAX_SHIFT];       // shift updated in this iteration
     int active_next[MS_MAX_SHIFT];  // after the freezing test
     double shift[MS_MAX_SHIFT];     // sigma_{r,i} - sigma_{r,0}: this RHS's poles relative to its base
-    // the scalars of each iteration m of the current window, for the delayed shifted updates:
-    // x_i -= h_om p_i, then p_i = h_ze r_m + h_ga p_i, applied by ms_flush_kernel when h_act
-    double h_om[MS_MAX_SHIFT][MS_WIN], h_ga[MS_MAX_SHIFT][MS_WIN], h_ze[MS_MAX_SHIFT][MS_WIN];
-    int h_act[MS_MAX_SHIFT][MS_WIN];
+};
+
+// the scalars of each iteration m of the current window, for the delayed shifted updates:
+// x_i -= om p_i, then p_i = ze r_m + ga p_i, applied by ms_flush_kernel when act
+struct MSHist {
+    double om[MS_MAX_SHIFT][MS_WIN], ga[MS_MAX_SHIFT][MS_WIN], ze[MS_MAX_SHIFT][MS_WIN];
+    int act[MS_MAX_SHIFT][MS_WIN];
 };
 
 struct MSState {
@@ -81,7 +86,9 @@ struct MSState {
     // is recomputed in FP64 from the FP64 base solution and the base direction re-synchronised
     int ru_every, ru_windows, ru_now, ru_count;
     MSRhs rhs[MS_MAX_RHS];
+    MSHist hist[MS_MAX_RHS];  // last: the host exchanges only what comes before it
 };
+constexpr size_t MS_STATE_HEAD = offsetof(MSState, hist);
 
 // ------------------------------------------------------------------ last-block scalar steps
 // The FP32 part of the precision schedule, with its FP64 reliable updates, leaves the shifted
@@ -155,6 +162,14 @@ struct FinInit {
     }
 };
 
+// zeta''' = zeta zeta'' omega_prev / (omega gamma (zeta - zeta'') + zeta omega_prev (1 - sigma omega)), rounded
+// one fixed way (see dot2), so that every kernel that steps it gives the same bits
+__device__ __forceinline__ double next_zeta(double zi, double zii, double omp, double om, double ga, double sh)
+{
+    return __dmul_rn(__dmul_rn(zi, zii), omp) /
+           dot2(__dmul_rn(om, ga), zi - zii, __dmul_rn(zi, omp), __fma_rn(-sh, om, 1.0));
+}
+
 template <int NR>
 struct FinAlpha {
     MSState *st;
@@ -202,16 +217,16 @@ struct FinAlpha {
             if (!in) continue;
             MSRhs &q = st->rhs[r];
             const int run = s_run[r], act = run ? an : 0;
-            q.h_act[i][wp] = act;
+            st->hist[r].act[i][wp] = act;
             if (!run) continue;
             q.active[i] = act;
             if (!act) continue;
             const double om = s_om[r], omp = s_omp[r];
-            const double ziii = (zi * zii * omp) / (om * s_ga[r] * (zi - zii) + zi * omp * (1.0 - sh * om));
+            const double ziii = next_zeta(zi, zii, omp, om, s_ga[r], sh);
             q.zeta_iii[i] = ziii;
             const double oms = om * ziii / zii;
             q.omegas[i] = oms;
-            q.h_om[i][wp] = oms;
+            st->hist[r].om[i][wp] = oms;
         }
     }
 };
@@ -270,8 +285,8 @@ struct FinLambda {
             MSRhs &q = st->rhs[r];
             const double gas = s_ga[r] * ziii * oms / (zii * s_om[r]);
             q.gammas[i] = gas;
-            q.h_ga[i][wp] = gas;
-            q.h_ze[i][wp] = ziii;
+            st->hist[r].ga[i][wp] = gas;
+            st->hist[r].ze[i][wp] = ziii;
             const double fact = sqrt(s_de[r] * zii * zii);
             const int an = (fact < tgt) ? 0 : 1;
             q.active_next[i] = an;
@@ -496,9 +511,9 @@ __global__ void __launch_bounds__(VEC_BLOCK, 2) ms_flush_kernel(int Vh, int nshi
         if (j < NR) {
             int any = 0, an = 0;
             if (i < nshift) {
-                const MSRhs &q = st->rhs[j];
+                const MSHist &hq = st->hist[j];
                 double2 *cf = s_coef + (size_t)j * rstride + i * (MS_WIN + 1);
-                an = q.active_next[i];
+                an = st->rhs[j].active_next[i];
                 double D = 0.0, G = 1.0;
                 // the window's scalars loaded in batches (entries past wp or of frozen iterations are
                 // stale and not used): one L2 latency per batch instead of one per iteration
@@ -510,10 +525,10 @@ __global__ void __launch_bounds__(VEC_BLOCK, 2) ms_flush_kernel(int Vh, int nshi
                     int act[B];
 #pragma unroll
                     for (int m = 0; m < B; m++) {
-                        om[m] = q.h_om[i][m0 + m];
-                        ga[m] = q.h_ga[i][m0 + m];
-                        ze[m] = q.h_ze[i][m0 + m];
-                        act[m] = m0 + m < wp ? q.h_act[i][m0 + m] : 0;
+                        om[m] = hq.om[i][m0 + m];
+                        ga[m] = hq.ga[i][m0 + m];
+                        ze[m] = hq.ze[i][m0 + m];
+                        act[m] = m0 + m < wp ? hq.act[i][m0 + m] : 0;
                     }
 #pragma unroll
                     for (int m = B - 1; m >= 0; m--) {

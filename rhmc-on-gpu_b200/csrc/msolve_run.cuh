@@ -10,6 +10,7 @@
 #include "context.h"
 #include "kernels.h"
 #include "msolve.cuh"
+#include "msolve_small.cuh"
 #include "solver.h"
 
 namespace rhmc {
@@ -19,17 +20,65 @@ static inline int vec_grid(rhmc_ctx *c) { return grid_for(c->Vh, VEC_BLOCK); }
 // workspace slot name of a base vector set in elements of `bytes` bytes
 static inline std::string vname(const char *base, size_t bytes) { return std::string(base) + std::to_string(bytes); }
 
-// Iterations per window of a phase whose residual ring takes `slot` bytes per iteration: MS_WIN when
-// the ring is already that long or fits with room to spare for what the rest of a solve may still
-// allocate (true residuals 16, refinement at most 52 FP64 spinors of v64 bytes), else half of it.
-static inline int ms_window(rhmc_ctx *c, const std::string &name, size_t slot, size_t v64)
+// The host's part of the initial state (what precedes MSState::hist); false when some right-hand
+// side does not iterate on one of its own poles.
+static inline bool ms_fill(const MSolveArgs &A, MSState &h0)
+{
+    memset(&h0, 0, MS_STATE_HEAD);
+    h0.nshift = A.nshift;
+    h0.nrhs = A.nrhs;
+    h0.max_iter = A.max_iter;
+    h0.stop_on_frozen = A.stop_on_frozen;
+    h0.res = A.res_base;
+    h0.tau = A.tau;
+    h0.first = 1;
+    h0.b = (const double2 *)A.b;
+    for (int i = 0; i < A.nshift; i++) h0.tgt[i] = A.tgt[i];
+    bool own = true;
+    for (int r = 0; r < A.nrhs; r++) {
+        int i0 = -1;
+        for (int i = 0; i < A.nshift; i++) {
+            h0.rhs[r].shift[i] = A.shift[(size_t)r * A.nshift + i] - A.base[r];
+            if (i0 < 0 && A.shift[(size_t)r * A.nshift + i] == A.base[r]) i0 = i;
+        }
+        own = own && i0 >= 0;
+        h0.rhs[r].i0 = i0 < 0 ? 0 : i0;
+    }
+    return own;
+}
+
+// What a finished phase left in the state (its head) into info; the phase's return code.
+static inline int ms_result(const MSState &hs, const MSolveArgs &A, MSolveInfo *info)
+{
+    if (info) {
+        info->status = hs.status;
+        info->ru_count = hs.ru_count;
+        for (int j = 0; j < A.nrhs; j++) {
+            info->iters[j] = hs.rhs[j].iter;
+            info->lambda[j] = hs.rhs[j].lambda;
+            info->b2[j] = hs.rhs[j].b2;
+        }
+    }
+    if (hs.status == 3) return fail(RHMC_ERR_CUDA, "multi-shift CG: a grid barrier timed out");
+    if (hs.status == 2) return fail(RHMC_ERR_NONFINITE, "multi-shift CG: non-finite reduction");
+    if (hs.status == 1) return fail(RHMC_ERR_MAXITER, "multi-shift CG: iteration cap %d reached", A.max_iter);
+    return RHMC_OK;
+}
+
+// The residual ring of a phase, `slot` bytes per iteration, and the iterations per window it allows:
+// MS_WIN when the ring is already that long, small (the query of free memory costs a new context's
+// first solve a millisecond or more) or fits with room to spare for what the rest of a solve may
+// still allocate (true residuals 16, refinement at most 52 FP64 spinors of v64 bytes), else half.
+static inline cudaError_t ms_ring(rhmc_ctx *c, const std::string &name, size_t slot, size_t v64, void **ring, int *win)
 {
     const auto it = c->ws.buf.find(name);
-    const size_t have = it == c->ws.buf.end() ? 0 : it->second.second;
-    if (have >= MS_WIN * slot) return MS_WIN;
-    size_t free_bytes = 0, total = 0;
-    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) return MS_WIN / 2;
-    return free_bytes + have >= MS_WIN * slot + 68 * v64 ? MS_WIN : MS_WIN / 2;
+    const size_t have = it == c->ws.buf.end() ? 0 : it->second.second, want = MS_WIN * slot;
+    *win = MS_WIN;
+    if (have < want && want + 68 * v64 > ((size_t)1 << 28)) {
+        size_t free_bytes = 0, total = 0;
+        if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || free_bytes + have < want + 68 * v64) *win = MS_WIN / 2;
+    }
+    return c->ws.get(name, *win * slot, ring);
 }
 
 // One phase of the multi-shift CG with links LF: base vectors (residual ring, p, h, s) in the
@@ -59,38 +108,20 @@ static int ms_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *
     CK(c->ws.get("ms_partials", (size_t)red_chunks(Vh) * 2 * NR * sizeof(double), &part));
     CK(c->ws.get("ms_tickets", 8 * sizeof(unsigned), &tick));
     // ring of the window's residuals [slot][rhs]
-    const int win = ms_window(c, vname("ms_r", sizeof(E)), NR * vbytes, v64);
-    CK(c->ws.get(vname("ms_r", sizeof(E)), (size_t)win * NR * vbytes, &r));
+    int win;
+    CK(ms_ring(c, vname("ms_r", sizeof(E)), NR * vbytes, v64, &r, &win));
     const int ru_every = (A.ru_every + win - 1) / win;  // in windows
     MSState *st = (MSState *)stv;
     unsigned *tk = (unsigned *)tick;
     double *pt = (double *)part;
     double2 *xs = (double2 *)A.x;
+    CK(cudaMemsetAsync(tk, 0, 8 * sizeof(unsigned), s_));
 
     if (A.fresh) {
         MSState h0;
-        memset(&h0, 0, sizeof(h0));
-        h0.nshift = S;
-        h0.nrhs = NR;
-        h0.max_iter = A.max_iter;
-        h0.stop_on_frozen = A.stop_on_frozen;
-        h0.res = A.res_base;
-        h0.tau = A.tau;
+        if (!ms_fill(A, h0) && ru) return fail(RHMC_ERR_ARG, "multi-shift: reliable updates need the base shift among the poles");
         h0.ru_every = ru_every;
-        for (int i = 0; i < S; i++) h0.tgt[i] = A.tgt[i];
-        for (int rr = 0; rr < NR; rr++) {
-            int i0 = -1;  // the pole the RHS iterates on (reliable updates need it among the poles)
-            for (int i = 0; i < S; i++) {
-                h0.rhs[rr].shift[i] = A.shift[(size_t)rr * S + i] - A.base[rr];
-                if (i0 < 0 && A.shift[(size_t)rr * S + i] == A.base[rr]) i0 = i;
-            }
-            if (ru && i0 < 0) return fail(RHMC_ERR_ARG, "multi-shift: reliable updates need the base shift among the poles");
-            h0.rhs[rr].i0 = i0 < 0 ? 0 : i0;
-        }
-        h0.wpos = 0;
-        h0.b = (const double2 *)A.b;
-        CK(cudaMemcpyAsync(st, &h0, sizeof(MSState), cudaMemcpyHostToDevice, s_));
-        CK(cudaMemsetAsync(tk, 0, 8 * sizeof(unsigned), s_));
+        CK(cudaMemcpyAsync(st, &h0, MS_STATE_HEAD, cudaMemcpyHostToDevice, s_));
         ms_init_kernel<Rv, NR><<<gv, VEC_BLOCK, 0, s_>>>(Vh, stride, win, (const double2 *)A.b, (E *)r, (E *)p, pt, tk, st);
         c->launches++;
         CK(cudaGetLastError());
@@ -229,25 +260,114 @@ static int ms_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *
     if (prc) return prc;
 
     MSState hs;
-    CK(cudaMemcpy(&hs, st, sizeof(MSState), cudaMemcpyDeviceToHost));
-    if (info) {
-        info->status = hs.status;
-        info->graph_replays += launched;
-        info->ru_count = hs.ru_count;
-        for (int j = 0; j < NR; j++) {
-            info->iters[j] = hs.rhs[j].iter;
-            info->lambda[j] = hs.rhs[j].lambda;
-            info->b2[j] = hs.rhs[j].b2;
-        }
+    CK(cudaMemcpy(&hs, st, MS_STATE_HEAD, cudaMemcpyDeviceToHost));
+    if (info) info->graph_replays += launched;
+    return ms_result(hs, A, info);
+}
+
+// ------------------------------------------------------------------ small lattices
+// Blocks of ms_small_kernel<LF, NR, MINB> that can be resident at once (0 when the query fails).
+template <class LF, int NR, int MINB>
+static long ms_small_capacity(int device, size_t smem)
+{
+    int occ = 0, sms = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ms_small_kernel<LF, NR, MINB>, MS_SMALL_BLOCK, smem) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
     }
-    if (hs.status == 2) return fail(RHMC_ERR_NONFINITE, "multi-shift CG: non-finite reduction");
-    if (hs.status == 1) return fail(RHMC_ERR_MAXITER, "multi-shift CG: iteration cap %d reached", A.max_iter);
-    return RHMC_OK;
+    return (long)occ * sms;
+}
+
+template <class LF, int NR, int MINB>
+static int ms_small_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *info)
+{
+    typedef typename LF::real Rv;
+    typedef typename SpinorT<Rv>::elem E;
+    cudaStream_t s_ = c->stream;
+    const int Vh = (int)c->Vh, n = A.nrhs;
+    const size_t stride = 3 * (size_t)Vh, vbytes = stride * sizeof(E), v64 = stride * sizeof(double2);
+    void *r, *p, *h, *q, *ps, *stv, *slots;
+    CK(c->ws.get(vname("ms_p", sizeof(E)), n * vbytes, &p));
+    CK(c->ws.get(vname("ms_h", sizeof(E)), n * vbytes, &h));
+    CK(c->ws.get(vname("ms_s", sizeof(E)), n * vbytes, &q));
+    CK(c->ws.get("ms_ps", (size_t)n * A.nshift * v64, &ps));
+    CK(c->ws.get("ms_state", sizeof(MSState), &stv));
+    const int nch = grid_for(Vh, MS_SMALL_BLOCK);
+    const size_t slot_bytes = (size_t)(n / NR) * 3 * ms_small_slots(NR, nch) * sizeof(ulonglong2);
+    CK(c->ws.get("ms_slots", slot_bytes, &slots));
+    int win;
+    CK(ms_ring(c, vname("ms_r", sizeof(E)), n * vbytes, v64, &r, &win));
+    MSState *st = (MSState *)stv;
+
+    MSState hs;
+    ms_fill(A, hs);
+    CK(cudaMemcpyAsync(st, &hs, MS_STATE_HEAD, cudaMemcpyHostToDevice, s_));
+    MSSmallArgs<LF> a;
+    a.g = c->g;
+    a.links = lf;
+    a.ring = (E *)r;
+    a.p = (E *)p;
+    a.q = (E *)q;
+    a.h = (E *)h;
+    a.ps = (double2 *)ps;
+    a.x = (double2 *)A.x;
+    a.slots = (ulonglong2 *)slots;
+    a.st = st;
+    a.nch = nch;
+    a.nshift = A.nshift;
+    a.nrhs = n;
+    a.win = win;
+    a.iters = MS_SMALL_ITERS;
+    a.init = 1;
+    for (int j = 0; j < MS_MAX_RHS; j++) a.alpha[j] = (Rv)(c->mass * c->mass + A.base[j < n ? j : 0]);
+    const size_t smem = ms_small_smem(NR, A.nshift);
+    for (int any = 1; any;) {
+        CK(cudaMemsetAsync(slots, 0, slot_bytes, s_));
+        void *args[] = {&a};
+        CK(cudaLaunchCooperativeKernel((const void *)ms_small_kernel<LF, NR, MINB>, dim3((unsigned)(a.nch * (n / NR))),
+                                       dim3(MS_SMALL_BLOCK), args, smem, s_));
+        c->launches++;
+        CK(cudaMemsetAsync(&st->first, 0, sizeof(int), s_));
+        CK(cudaMemcpyAsync(&hs, st, MS_STATE_HEAD, cudaMemcpyDeviceToHost, s_));
+        CK(cudaStreamSynchronize(s_));
+        a.init = 0;
+        any = 0;
+        for (int j = 0; j < n; j++) any |= hs.rhs[j].running_next;
+        if (hs.status >= 2) any = 0;
+    }
+    return ms_result(hs, A, info);
+}
+
+// Runs a fresh phase as one kernel when all its blocks, one per 128 sites and right-hand side, fit on
+// the device at once; false when they do not.  Two resident blocks per SM leave the kernel 255
+// registers and its neighbour loads in larger batches (4 directions of p and r; 16.1 against
+// 17.2 us an iteration on 12^3x24), three (168 registers) take half as many blocks again; then a
+// block carries two right-hand sides, which reads the links once for both.  Every size that fits
+// is faster than the launches it replaces, us an iteration: 4^4 6.4 against 21, 8^4 11 against 21,
+// 12^4 12.9 against 21, 12^3x24 two right-hand sides 20 against 29, 16^4 one 18 against 26 and two
+// 24 against 32, 16^3x26 one 24 against 31 (FP64, 8 to 15 poles).
+template <class LF>
+static bool ms_small(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *info, int *rc)
+{
+    const long chunks = grid_for(c->Vh, MS_SMALL_BLOCK);
+    const size_t s1 = ms_small_smem(1, A.nshift), s2 = ms_small_smem(2, A.nshift);
+    if (chunks * A.nrhs <= ms_small_capacity<LF, 1, 2>(c->device, s1))
+        *rc = ms_small_phase<LF, 1, 2>(c, lf, A, info);
+    else if (chunks * A.nrhs <= ms_small_capacity<LF, 1, 3>(c->device, s1))
+        *rc = ms_small_phase<LF, 1, 3>(c, lf, A, info);
+    else if (A.nrhs % 2 == 0 && chunks * (A.nrhs / 2) <= ms_small_capacity<LF, 2, 2>(c->device, s2))
+        *rc = ms_small_phase<LF, 2, 2>(c, lf, A, info);
+    else
+        return false;
+    return true;
 }
 
 template <class LF>
 int ms_run(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *info)
 {
+    int rc = RHMC_OK;
+    if (A.fresh && A.ru_every == 0 && ms_small<LF>(c, lf, A, info, &rc)) return rc;
     switch (A.nrhs) {
     case 1: return ms_phase<LF, 1>(c, lf, A, info);
     case 2: return ms_phase<LF, 2>(c, lf, A, info);
