@@ -95,8 +95,11 @@ __global__ void __launch_bounds__(BLOCK, MINB) dslash_kernel(DslashArgs<LF, NR, 
     typedef typename S::elem E;
     // tiles of BLOCK consecutive output sites; a launch with fewer blocks than tiles (persistent
     // blocks) walks them with stride gridDim.x, so the per-block work of the fused reduction
-    // (fence, ticket) is paid once per block instead of once per tile
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    // (fence, ticket) is paid once per block instead of once per tile.  Launches onto the even sites
+    // walk the tiles downwards and those onto the odd sites upwards (and the solvers' vector kernels
+    // alternate likewise), so a launch starts on what the one before it left in L2.
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const int tile = a.p_out == 0 ? ntiles - 1 - t : t;
         const int k = a.k_lo + tile * BLOCK + threadIdx.x;
         if constexpr (S::pack > 1) {
             // packed right-hand sides: one load brings P of them (PackS)

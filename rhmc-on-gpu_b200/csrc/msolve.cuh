@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(VEC_BLOCK) ms_update_kernel(int Vh, size_t str
     typedef PackIO<Rv, P> IO;
     typedef PackElem<Rv, P> PE;
     if (*(volatile int *)&st->stop_k4) return;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;  // downwards, K3 went upwards
     if (k >= Vh) return;
     const E *r = ring + (size_t)(*(volatile const int *)&st->wpos - 1) * NR * stride;  // K3 advanced wpos
 #pragma unroll

@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(VEC_BLOCK) rb_p_kernel(int Vh, size_t sstride,
 {
     typedef typename S::real Rs;
     if (*(volatile const int *)&st->stop) return;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;  // downwards, rb_xr_kernel went upwards
     if (k >= Vh) return;
 #pragma unroll
     for (int j = 0; j < NR; j++) {
