@@ -69,12 +69,16 @@ __global__ void __launch_bounds__(UPD_BLOCK) link_update_kernel(Geom g, double2 
 // read for three planes each (L1 hits); warps alternate between the parities, as in force.cu, so
 // that links read as neighbours come from L2.  32^4: 213 us (471 us with three products a plane,
 // formed with separate additions, and three threads a site); 230 us with three threads a site,
-// 238 us at 16 warps per SM; the HBM floor is 93 us, the FP64 floor 87 us.
+// 238 us at 16 warps per SM; the HBM floor is 93 us, the FP64 floor 87 us.  Lattices whose sites fill
+// at most one wave of blocks are bound by the chain of six planes instead: there each block takes
+// one plane, the plane as the fastest block index (split = 6 instead of 1).
 constexpr int PLAQ_BLOCK = 128;
+constexpr int PLAQ_RESIDENT = 3;  // blocks per SM
 
-__global__ void __launch_bounds__(PLAQ_BLOCK, 3) plaq_kernel(Geom g, const double2 *__restrict__ U, double *partials)
+__global__ void __launch_bounds__(PLAQ_BLOCK, PLAQ_RESIDENT) plaq_kernel(Geom g, const double2 *__restrict__ U, double *partials, int split)
 {
-    const long chunk = (long)blockIdx.x * (PLAQ_BLOCK / 32) + (threadIdx.x >> 5);
+    const long chunk = (long)(blockIdx.x / split) * (PLAQ_BLOCK / 32) + (threadIdx.x >> 5);
+    const int pl0 = split == 1 ? 0 : blockIdx.x % split, pl1 = split == 1 ? 6 : pl0 + 1;
     const int Vh = g.Vh;
     const int p = (int)(chunk & 1), q = 1 - p;
     const long k0 = (chunk >> 1) * 32 + (threadIdx.x & 31);
@@ -83,7 +87,7 @@ __global__ void __launch_bounds__(PLAQ_BLOCK, 3) plaq_kernel(Geom g, const doubl
         const int k = (int)k0;
         const Site s = site_of(g, p, k);
 #pragma unroll 1
-        for (int pl = 0; pl < 6; pl++) {
+        for (int pl = pl0; pl < pl1; pl++) {
             const int mu = pl < 3 ? 0 : (pl < 5 ? 1 : 2), nu = pl < 3 ? pl + 1 : (pl < 5 ? pl - 1 : 3);
             const M3 A = load_link64(U, Vh, nu, q, neighbour(g, s, mu, +1));
             const M3 B = load_link64(U, Vh, mu, q, neighbour(g, s, nu, +1));
@@ -184,20 +188,17 @@ __global__ void __launch_bounds__(SUM_BLOCK) sum_partials_kernel(const double *_
         for (int j = 0; j < N; j++) out[j] = v[j];
 }
 
-// The N sums of nblocks per-block partials, read back through the context's pinned words (behind
-// the solver's polling words).  Summing on the device leaves 8 N bytes to copy; copying every partial
-// to pageable memory and adding them on the host cost 30-60 us per call at 32^4.
+// The N sums of nblocks per-block partials.  One block adds them on the device and stores the sums
+// into the context's pinned words (behind the solver's polling words), so nothing is copied: copying
+// every partial to pageable memory and adding them on the host cost 30-60 us per call at 32^4.
 template <int N>
 static int read_sums(rhmc_ctx *c, const double *dpart, int nblocks, double *out)
 {
     static_assert(N <= 8, "pinned words hold 8 doubles past the polling words");
-    void *tot;
-    CK(c->ws.get("red_tot", 8 * sizeof(double), &tot));
-    sum_partials_kernel<N><<<1, SUM_BLOCK, 0, c->stream>>>(dpart, nblocks, (double *)tot);
+    double *h = reinterpret_cast<double *>(c->hflags) + 8;  // 64 bytes into the 256 pinned ones
+    sum_partials_kernel<N><<<1, SUM_BLOCK, 0, c->stream>>>(dpart, nblocks, h);
     c->launches++;
     CK(cudaGetLastError());
-    double *h = reinterpret_cast<double *>(c->hflags) + 8;  // 64 bytes into the 256 pinned ones
-    CK(cudaMemcpyAsync(h, tot, N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     for (int j = 0; j < N; j++) out[j] = h[j];
     return RHMC_OK;
@@ -223,10 +224,12 @@ int link_update(rhmc_ctx *c, double step)
 // sums over all sites of ReTr(plaquette): temporal (nu = 3) and spatial
 int plaquette_sums(rhmc_ctx *c, double *temporal, double *spatial)
 {
-    const int nb = grid_for(2L * grid_for(c->Vh, 32), PLAQ_BLOCK / 32);  // a warp per 32 half-sites
+    const int sites = grid_for(2L * grid_for(c->Vh, 32), PLAQ_BLOCK / 32);  // blocks; a warp per 32 half-sites
+    const int split = sites <= PLAQ_RESIDENT * 148 ? 6 : 1;
+    const int nb = sites * split;
     void *part;
     CK(c->ws.get("red_part", (size_t)nb * 2 * sizeof(double), &part));
-    plaq_kernel<<<nb, PLAQ_BLOCK, 0, c->stream>>>(c->g, c->U64, (double *)part);
+    plaq_kernel<<<nb, PLAQ_BLOCK, 0, c->stream>>>(c->g, c->U64, (double *)part, split);
     c->launches++;
     CK(cudaGetLastError());
     double o[2] = {0.0, 0.0};
