@@ -78,9 +78,9 @@ static int refine_all(rhmc_ctx *c, const LF &lf, int nshift, const double *shift
             CK(cudaMemcpyAsync((double2 *)bg + j * stride, b + (size_t)(q / nshift) * stride, v64, cudaMemcpyDeviceToDevice,
                                c->stream));
         }
-        // iterations between reliable-update stages (systems that need none skip the stage)
-        const double kappa = (16.0 + coef[0]) / coef[0];
-        const int n_ru = kappa > 1e3 ? 16 : 8;
+        // iterations between reliable-update stages: a waiting system idles until the next one, and the
+        // stage costs a system that needs none only its skipped launches
+        const int n_ru = 8;
         int rc = rb_group_n(c, lf, n, coef, tgt, (double2 *)xg, (const double2 *)bg, max_iter, n_ru, iters, ru, ru_delta);
         if (rc) return rc;
         for (int j = 0; j < n; j++) {

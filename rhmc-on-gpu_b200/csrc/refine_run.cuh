@@ -21,6 +21,8 @@ struct ResidCoef {
     double coef[8];  // mass^2 + sigma of each batched system
 };
 
+constexpr double RB_MARGIN = 0.25;
+
 struct RBState {
     int stop;         // every system converged (or failed)
     int status;       // 0 ok, 2 non-finite
@@ -162,9 +164,11 @@ struct FinRBBeta {
             st->beta[j] = (st->rr[j] > 0.0) ? rn / st->rr[j] : 0.0;
             st->rr[j] = rn;
             st->since[j]++;
-            // update after a drop by delta, after ru_max iterations, or when the FP32 iteration
-            // stops making progress (its residual above 4x the last true one)
-            if (rn <= st->delta2 * st->rr_ru[j] || st->since[j] >= st->ru_max || !isfinite(rn) || rn > 4.0 * st->rr_ru[j]) {
+            // update after a drop by delta, once below the target (with RB_MARGIN for the true residual
+            // to be there too; most systems start a few times above it and would otherwise be iterated
+            // on to delta), after ru_max iterations, or when the FP32 iteration stops making progress
+            // (its residual above 4x the last true one)
+            if (rn <= st->delta2 * st->rr_ru[j] || rn <= RB_MARGIN * RB_MARGIN * st->tgt[j] * st->tgt[j] || st->since[j] >= st->ru_max || !isfinite(rn) || rn > 4.0 * st->rr_ru[j]) {
                 st->pending[j] = 1;
                 st->any_pending = 1;
             }
