@@ -8,10 +8,10 @@
 //                        (lib/Action/fermionforce.cc:46-104): even x: sum a_i h_i(x+mu) (x) x_i(x)^*,
 //                        odd x: -sum a_i x_i(x+mu) (x) h_i(x)^*, h_i = Doe x_i (with its 1/2).
 // gauge_force_kernel runs one thread per site and mu (a warp per mu);
-// fermion_force_kernel one thread per link, mu fastest inside a site (the four links of a site
-// share the site's spinor loads through L1).  All shifted solutions of all right-hand sides are summed in registers,
-// so the 18-real force matrix never goes to HBM (the reference GPU code read-modify-writes an
-// 18 x 4V float buffer once per shift, lib/Cuda/cuda_fermion_force.cu:370-386).
+// fermion_force_kernel one thread per site and one or two mu.  All shifted solutions of all
+// right-hand sides are summed in registers, so the 18-real force matrix never goes to HBM (the
+// reference GPU code read-modify-writes an 18 x 4V float buffer once per shift,
+// lib/Cuda/cuda_fermion_force.cu:370-386).
 #include <string>
 #include <vector>
 
@@ -93,8 +93,7 @@ __device__ M3 staple_sum(const Geom &g, const double2 *__restrict__ U, int mu, i
 // neighbour, by the threads of the other parity: in a parity-major order those two reads lie a
 // whole half-lattice apart, which at 24^4 and above is more than L2 holds, and every such
 // element came from HBM twice.
-constexpr int GF_CHUNK = 32;  // half-sites per warp, gauge force
-constexpr int FF_CHUNK = 8;   // half-sites per warp (x 4 mu), fermion force
+constexpr int GF_CHUNK = 32;  // half-sites per warp
 
 __host__ __device__ __forceinline__ long force_chunks(int Vh, int W) { return 2L * ((Vh + W - 1) / W); }
 
@@ -134,60 +133,79 @@ __global__ void __launch_bounds__(FORCE_BLOCK, 3) gauge_force_kernel(Geom g, con
     store_alg(IP, Vh, mu, p, k, o);
 }
 
-// x: even FP64 spinors [nv], h = Doe x: odd FP64 spinors [nv]; coef[v] the numerator of vector v.
-// UNR vectors are unrolled (their loads issued together) and MINB blocks are kept resident per
-// SM; the kernel waits on its loads more than on its FMAs, so the pair that keeps most bytes in
-// flight wins, and the autotuner picks it per volume and vector count (FF_SHAPES).
-template <int UNR, int MINB>
+// x: even FP64 spinors [nv], h = Doe x: odd FP64 spinors; coef[v] the numerator of vector v.
+// A warp covers 32 consecutive half-sites of one parity and NMU directions (a block: the directions of
+// a chunk, then the next chunk), so a vector's loads of a warp are contiguous 512-byte segments.
+// Bound by the L2 traffic of the neighbours' vectors (each site's vector is wanted by four other
+// sites) and its latency.  NMU = 2 loads the site's own vector once for two directions and keeps two
+// force matrices in registers; NMU = 1 keeps more warps in flight, which small lattices need.  30
+// vectors at 24^3x32: 330 us with NMU = 2 at four blocks per SM, 348 us with NMU = 1, 407 us for a
+// warp of 8 sites x 4 directions (the HBM floor is 155 us).  UNR vectors are unrolled (their loads
+// issued together) and MINB blocks kept resident; the autotuner picks per volume and vector count
+// (FF_SHAPES).
+template <int NMU, int UNR, int MINB>
 __global__ void __launch_bounds__(FORCE_BLOCK, MINB) fermion_force_kernel(Geom g, const double2 *__restrict__ U,
                                                                            const double2 *__restrict__ x,
                                                                            const double2 *__restrict__ h, int nv,
                                                                            const double *__restrict__ coef, double *IP,
                                                                            int mode)
 {
-    // a warp: FF_CHUNK half-sites of one parity x 4 mu, mu the fastest thread index
-    const int Vh = g.Vh;
-    const long chunk = (long)blockIdx.x * (FORCE_BLOCK / 32) + (threadIdx.x >> 5);
-    if (chunk >= force_chunks(Vh, FF_CHUNK)) return;
-    const int mu = threadIdx.x & 3;
+    constexpr int WARPS = 4 / NMU;  // warps per chunk
+    const int Vh = g.Vh, wid = threadIdx.x >> 5;
+    const long chunk = (long)blockIdx.x * (FORCE_BLOCK / 32 / WARPS) + wid / WARPS;
+    if (chunk >= force_chunks(Vh, GF_CHUNK)) return;
+    const int mu0 = (wid % WARPS) * NMU;
     const int p = (int)(chunk & 1);
-    const int k = (int)(chunk >> 1) * FF_CHUNK + ((threadIdx.x & 31) >> 2);
+    const int k = (int)(chunk >> 1) * GF_CHUNK + (threadIdx.x & 31);
     if (k >= Vh) return;
     const Site s = site_of(g, p, k);
-    const int kn = neighbour(g, s, mu, +1);  // x+mu, opposite parity
+    int kn[NMU];  // x+mu, opposite parity
+#pragma unroll
+    for (int m = 0; m < NMU; m++) kn[m] = neighbour(g, s, mu0 + m, +1);
     const size_t stride = 3 * (size_t)Vh;
     // even x: a h(x+mu) (x) x(x)^* ; odd x: -a x(x+mu) (x) h(x)^*
     const double2 *left = p == 0 ? h : x;
     const double2 *right = p == 0 ? x : h;
-    const int kl = kn, kr = k;
     const double sgn = p == 0 ? 1.0 : -1.0;
-    M3 F = m3_zero();
+    M3 F[NMU];
+#pragma unroll
+    for (int m = 0; m < NMU; m++) F[m] = m3_zero();
 #pragma unroll UNR
     for (int v = 0; v < nv; v++) {
         const double a = sgn * __ldg(coef + v);
         const double2 *L = left + v * stride, *R = right + v * stride;
-        C l[3], r[3];
+        C l[NMU][3], r[3];
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-            const double2 lv = __ldg(L + (size_t)c * Vh + kl), rv = __ldg(R + (size_t)c * Vh + kr);
-            l[c] = mk<double>(a * lv.x, a * lv.y);
-            r[c] = mk<double>(rv.x, -rv.y);
+            const double2 rv = __ldg(R + (size_t)c * Vh + k);
+            r[c] = mk<double>(a * rv.x, -a * rv.y);
+#pragma unroll
+            for (int m = 0; m < NMU; m++) {
+                const double2 lv = __ldg(L + (size_t)c * Vh + kn[m]);
+                l[m][c] = mk<double>(lv.x, lv.y);
+            }
         }
 #pragma unroll
-        for (int i = 0; i < 3; i++)
+        for (int m = 0; m < NMU; m++)
 #pragma unroll
-            for (int j = 0; j < 3; j++) F.e[i][j] = cmadd(l[i], r[j], F.e[i][j]);
-    }
-    const M3 uf = m3_mul(load_link64(U, Vh, mu, p, k), F);
-    double o[8];
-    ta_pack(uf, o);
-    if (mode) {
-        double c[8];
-        load_alg(IP, Vh, mu, p, k, c);
+            for (int i = 0; i < 3; i++)
 #pragma unroll
-        for (int j = 0; j < 8; j++) o[j] += c[j];
+                for (int j = 0; j < 3; j++) F[m].e[i][j] = cmadd(l[m][i], r[j], F[m].e[i][j]);
     }
-    store_alg(IP, Vh, mu, p, k, o);
+#pragma unroll
+    for (int m = 0; m < NMU; m++) {
+        const int mu = mu0 + m;
+        const M3 uf = m3_mul(load_link64(U, Vh, mu, p, k), F[m]);
+        double o[8];
+        ta_pack(uf, o);
+        if (mode) {
+            double c[8];
+            load_alg(IP, Vh, mu, p, k, c);
+#pragma unroll
+            for (int j = 0; j < 8; j++) o[j] += c[j];
+        }
+        store_alg(IP, Vh, mu, p, k, o);
+    }
 }
 
 int gauge_force(rhmc_ctx *c, int mode)
@@ -199,20 +217,28 @@ int gauge_force(rhmc_ctx *c, int mode)
     return RHMC_OK;
 }
 
-// (vectors unrolled, minimum resident blocks per SM) of the fermion force's launch candidates;
-// candidate 0 is the default when tuning is off
+// (directions per thread, vectors unrolled, minimum resident blocks per SM) of the fermion force's
+// launch candidates; candidate 0 is the default when tuning is off
 constexpr int FF_NCAND = 4;
-constexpr int FF_SHAPES[FF_NCAND][2] = {{2, 1}, {4, 1}, {2, 6}, {4, 4}};
+constexpr int FF_SHAPES[FF_NCAND][3] = {{2, 1, 4}, {1, 2, 1}, {1, 4, 1}, {2, 2, 2}};
+
+template <int CAND>
+static void ff_launch_cand(const rhmc_ctx *c, const double2 *x, const double2 *h, int nv, const double *co, double *IP, int mode)
+{
+    constexpr int NMU = FF_SHAPES[CAND][0];
+    const unsigned grid = (unsigned)grid_for(force_chunks(c->Vh, GF_CHUNK), FORCE_BLOCK / 32 * NMU / 4);
+    fermion_force_kernel<NMU, FF_SHAPES[CAND][1], FF_SHAPES[CAND][2]><<<grid, FORCE_BLOCK, 0, c->stream>>>(c->g, c->U64, x, h, nv,
+                                                                                                          co, IP, mode);
+}
 
 static void ff_launch(int cand, const rhmc_ctx *c, const double2 *x, const double2 *h, int nv, const double *co,
                       double *IP, int mode)
 {
-    const unsigned grid = (unsigned)grid_for(force_chunks(c->Vh, FF_CHUNK), FORCE_BLOCK / 32);
     switch (cand) {
-    case 1: fermion_force_kernel<4, 1><<<grid, FORCE_BLOCK, 0, c->stream>>>(c->g, c->U64, x, h, nv, co, IP, mode); break;
-    case 2: fermion_force_kernel<2, 6><<<grid, FORCE_BLOCK, 0, c->stream>>>(c->g, c->U64, x, h, nv, co, IP, mode); break;
-    case 3: fermion_force_kernel<4, 4><<<grid, FORCE_BLOCK, 0, c->stream>>>(c->g, c->U64, x, h, nv, co, IP, mode); break;
-    default: fermion_force_kernel<2, 1><<<grid, FORCE_BLOCK, 0, c->stream>>>(c->g, c->U64, x, h, nv, co, IP, mode); break;
+    case 1: ff_launch_cand<1>(c, x, h, nv, co, IP, mode); break;
+    case 2: ff_launch_cand<2>(c, x, h, nv, co, IP, mode); break;
+    case 3: ff_launch_cand<3>(c, x, h, nv, co, IP, mode); break;
+    default: ff_launch_cand<0>(c, x, h, nv, co, IP, mode); break;
     }
 }
 
@@ -223,7 +249,7 @@ static int ff_candidate(rhmc_ctx *c, const double2 *x, const double2 *h, int nv,
 {
     if (autotune_override() >= 0) return autotune_override() < FF_NCAND ? autotune_override() : 0;
     if (!autotune_enabled()) return 0;
-    const std::string key = tune_key(c->Vh, "fermion_force nv=" + std::to_string(nv));
+    const std::string key = tune_key(c->Vh, "fermion_force 32-site nv=" + std::to_string(nv));
     const int got = tune_get(key);
     if (got >= 0) return got;
     if (stream_capturing(c->stream)) return 0;
@@ -248,7 +274,7 @@ static int ff_candidate(rhmc_ctx *c, const double2 *x, const double2 *h, int nv,
         for (int k = 1; k < FF_NCAND; k++)
             if (us[k] < us[best]) best = k;
         DsShape shapes[FF_NCAND];
-        for (int k = 0; k < FF_NCAND; k++) shapes[k] = DsShape{FORCE_BLOCK, FF_SHAPES[k][1]};
+        for (int k = 0; k < FF_NCAND; k++) shapes[k] = DsShape{FORCE_BLOCK, FF_SHAPES[k][2]};
         tune_put(key, best, us, shapes, FF_NCAND);
     } else {
         best = 0;
