@@ -266,12 +266,12 @@ static int ms_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *
 }
 
 // ------------------------------------------------------------------ small lattices
-// Blocks of ms_small_kernel<LF, NR, MINB> that can be resident at once (0 when the query fails).
+// Blocks of ms_small_kernel<LF, NR, MINB, false> that can be resident at once (0 when the query fails).
 template <class LF, int NR, int MINB>
 static long ms_small_capacity(int device, size_t smem)
 {
     int occ = 0, sms = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ms_small_kernel<LF, NR, MINB>, MS_SMALL_BLOCK, smem) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ms_small_kernel<LF, NR, MINB, false>, MS_SMALL_BLOCK, smem) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
         cudaGetLastError();
         return 0;
@@ -279,7 +279,40 @@ static long ms_small_capacity(int device, size_t smem)
     return (long)occ * sms;
 }
 
-template <class LF, int NR, int MINB>
+// The launch of `groups` clusters of nch blocks; the attribute lives in *attr.
+static inline cudaLaunchConfig_t ms_cluster_config(int nch, int groups, size_t smem, cudaStream_t s, cudaLaunchAttribute *attr)
+{
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = (unsigned)nch;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(nch * groups));
+    cfg.blockDim = dim3(MS_SMALL_BLOCK);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// Whether a cluster of nch blocks of the kernel can be scheduled on this device.
+template <class LF>
+static bool ms_cluster_fits(int nch, size_t smem)
+{
+    auto kern = ms_small_kernel<LF, 1, 2, true>;
+    if (nch > MS_CLUSTER) return false;
+    cudaLaunchAttribute attr;
+    cudaLaunchConfig_t cfg = ms_cluster_config(nch, 1, smem, nullptr, &attr);
+    int n = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return n >= 1;
+}
+
+template <class LF, int NR, int MINB, bool CL>
 static int ms_small_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *info)
 {
     typedef typename LF::real Rv;
@@ -325,8 +358,14 @@ static int ms_small_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolve
     for (int any = 1; any;) {
         CK(cudaMemsetAsync(slots, 0, slot_bytes, s_));
         void *args[] = {&a};
-        CK(cudaLaunchCooperativeKernel((const void *)ms_small_kernel<LF, NR, MINB>, dim3((unsigned)(a.nch * (n / NR))),
-                                       dim3(MS_SMALL_BLOCK), args, smem, s_));
+        const void *kern = (const void *)ms_small_kernel<LF, NR, MINB, CL>;
+        if (CL) {
+            cudaLaunchAttribute attr;
+            const cudaLaunchConfig_t cfg = ms_cluster_config(nch, n / NR, smem, s_, &attr);
+            CK(cudaLaunchKernelExC(&cfg, kern, args));
+        } else {
+            CK(cudaLaunchCooperativeKernel(kern, dim3((unsigned)(nch * (n / NR))), dim3(MS_SMALL_BLOCK), args, smem, s_));
+        }
         c->launches++;
         CK(cudaMemsetAsync(&st->first, 0, sizeof(int), s_));
         CK(cudaMemcpyAsync(&hs, st, MS_STATE_HEAD, cudaMemcpyDeviceToHost, s_));
@@ -344,7 +383,8 @@ static int ms_small_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolve
 // registers and its neighbour loads in larger batches (4 directions of p and r; 16.1 against
 // 17.2 us an iteration on 12^3x24), three (168 registers) take half as many blocks again; then a
 // block carries two right-hand sides, which reads the links once for both.  Every size that fits
-// is faster than the launches it replaces, us an iteration: 4^4 6.4 against 21, 8^4 11 against 21,
+// is faster than the launches it replaces, us an iteration: 4^4 6.4 against 21, 8^4 9.0 against 21
+// (as clusters; 10 to 13 when its 16 blocks meet through L2, depending on where they land),
 // 12^4 12.9 against 21, 12^3x24 two right-hand sides 20 against 29, 16^4 one 18 against 26 and two
 // 24 against 32, 16^3x26 one 24 against 31 (FP64, 8 to 15 poles).
 template <class LF>
@@ -352,12 +392,14 @@ static bool ms_small(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo 
 {
     const long chunks = grid_for(c->Vh, MS_SMALL_BLOCK);
     const size_t s1 = ms_small_smem(1, A.nshift), s2 = ms_small_smem(2, A.nshift);
-    if (chunks * A.nrhs <= ms_small_capacity<LF, 1, 2>(c->device, s1))
-        *rc = ms_small_phase<LF, 1, 2>(c, lf, A, info);
+    if (chunks > 1 && ms_cluster_fits<LF>((int)chunks, s1))
+        *rc = ms_small_phase<LF, 1, 2, true>(c, lf, A, info);
+    else if (chunks * A.nrhs <= ms_small_capacity<LF, 1, 2>(c->device, s1))
+        *rc = ms_small_phase<LF, 1, 2, false>(c, lf, A, info);
     else if (chunks * A.nrhs <= ms_small_capacity<LF, 1, 3>(c->device, s1))
-        *rc = ms_small_phase<LF, 1, 3>(c, lf, A, info);
+        *rc = ms_small_phase<LF, 1, 3, false>(c, lf, A, info);
     else if (A.nrhs % 2 == 0 && chunks * (A.nrhs / 2) <= ms_small_capacity<LF, 2, 2>(c->device, s2))
-        *rc = ms_small_phase<LF, 2, 2>(c, lf, A, info);
+        *rc = ms_small_phase<LF, 2, 2, false>(c, lf, A, info);
     else
         return false;
     return true;

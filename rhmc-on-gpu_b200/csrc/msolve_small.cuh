@@ -23,6 +23,8 @@
 // Co-residency: launched cooperatively; an exchange gives up after MS_SPIN_LIMIT polls, flags
 // MSState::status = 3 and every block leaves.
 #pragma once
+#include <cooperative_groups.h>
+
 #include "msolve.cuh"
 
 namespace rhmc {
@@ -32,6 +34,7 @@ constexpr unsigned MS_SPIN_LIMIT = 1u << 21;  // about a second
 constexpr int MS_SMALL_ITERS = 1024;  // iterations per launch (about 10 ms; whole windows)
 
 constexpr int MS_SLOT_CHUNKS = 32;
+constexpr int MS_CLUSTER = 16;  // largest group that runs as a cluster (the non-portable maximum)
 
 // entries of one kind of exchange of a group of nr right-hand sides: slots (or sums) and the counter
 __host__ __device__ inline size_t ms_small_slots(int nr, int nch) { return (size_t)nr * nch + 1; }
@@ -85,9 +88,11 @@ struct Meeting {
 };
 
 // Group-wide sums of N values per thread, in every thread of every block, added in the order of
-// reduce_tile and reduce_last.  With DATA every store before the exchange is also visible to the
+// reduce_tile and reduce_last (a zero added to a partial sum changes no bit).  With DATA every store before the exchange is also visible to the
 // loads after it (ld.cg) in all blocks of the group, i.e. it is the barrier as well; without, it
 // orders nothing but the sums.
+//   * up to MS_CLUSTER chunks: the group is a cluster, which meets at its hardware barrier and passes
+//     the sums through shared memory;
 //   * sums of up to MS_SLOT_CHUNKS chunks: every block publishes its chunk sums in slots that carry the
 //     number of the exchange and reads all chunks' slots until they do: one publication and one
 //     poll latency (8^4, 16 chunks: 2,200 to 3,900 cycles against 4,500 to 4,900 when counted);
@@ -110,18 +115,51 @@ __device__ __forceinline__ bool group_arrive(Meeting &w, MSState *st, int ok)
 }
 
 // the barrier alone
+template <bool CL>
 __device__ __forceinline__ bool group_barrier(Meeting &w, int nch, MSState *st)
 {
+    if constexpr (CL) {
+        cooperative_groups::this_cluster().sync();
+        return true;
+    }
     __syncthreads();
     w.target += nch;
     return nch == 1 || group_arrive(w, st, 1);
 }
 
-template <int N, bool DATA>
+template <int N, bool DATA, bool CL>
 __device__ __forceinline__ bool group_exchange(const double (&v)[N], double (&tot)[N], Meeting &w, int nch, int chunk, MSState *st)
 {
     __shared__ double sm[N][MS_SMALL_BLOCK];
     __shared__ double wsum[N][4];
+    if constexpr (CL) {
+        // every block's chunk sums into every block's shared memory, one array per kind of exchange (a
+        // block is past the next exchange's barrier only when all have read this one's)
+        __shared__ double peer[N][MS_CLUSTER];
+        namespace cg = cooperative_groups;
+        cg::cluster_group cl = cg::this_cluster();
+        const int ln = threadIdx.x & 31, wd = threadIdx.x >> 5;
+#pragma unroll
+        for (int j = 0; j < N; j++) sm[j][threadIdx.x] = v[j];
+        __syncthreads();
+        for (int j = wd; j < N; j += 4) {
+            double t = sm[j][ln];
+            t += sm[j][ln + 32];
+            t += sm[j][ln + 64];
+            t += sm[j][ln + 96];
+            t = warp_sum(t);
+            if (ln < nch) *cl.map_shared_rank(&peer[j][chunk], ln) = t;
+        }
+        cl.sync();
+        // the order of reduce_last: lane t holds chunk t (fewer than 128 chunks: one each), zeros beyond,
+        // a shuffle tree, and the sums of the three other warps, which are zero
+#pragma unroll
+        for (int j = 0; j < N; j++) {
+            double t = warp_sum(ln < nch ? peer[j][ln] : 0.0);
+            tot[j] = t;
+        }
+        return true;
+    }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const bool counted = nch > MS_SLOT_CHUNKS;
     double *part = reinterpret_cast<double *>(w.slots);
@@ -225,7 +263,8 @@ __device__ __forceinline__ void direction(vec3<R> &p, const vec3<R> &r, R g)
     }
 }
 
-template <class LF, int NR, int MINB>
+// CL: the group is a thread-block cluster of nch blocks
+template <class LF, int NR, int MINB, bool CL>
 __global__ void __launch_bounds__(MS_SMALL_BLOCK, MINB) ms_small_kernel(MSSmallArgs<LF> a)
 {
     typedef typename LF::real R;
@@ -289,7 +328,7 @@ __global__ void __launch_bounds__(MS_SMALL_BLOCK, MINB) ms_small_kernel(MSSmallA
                 stcg3<R>(a.ring + ((size_t)(a.win - 1) * a.nrhs + r0 + j) * stride, Vh, k, r[j]);
             }
         }
-        if (!group_exchange<NR, true>(red, tot, meet[2], nch, chunk, st)) return;
+        if (!group_exchange<NR, true, CL>(red, tot, meet[2], nch, chunk, st)) return;
         const double rs = st->res, tau = st->tau;
 #pragma unroll
         for (int j = 0; j < NR; j++) {
@@ -335,7 +374,7 @@ __global__ void __launch_bounds__(MS_SMALL_BLOCK, MINB) ms_small_kernel(MSSmallA
             an = q.active_next[lane];
         }
         // every block has read the state before one of the group writes it at the end
-        if (!group_barrier(meet[2], nch, st)) return;
+        if (!group_barrier<CL>(meet[2], nch, st)) return;
     }
     E *pc = a.p, *pn = a.q;  // current and next direction buffer
     int wp = 0;
@@ -504,7 +543,7 @@ __global__ void __launch_bounds__(MS_SMALL_BLOCK, MINB) ms_small_kernel(MSSmallA
         }
 #pragma unroll
         for (int j = 0; j < NR; j++) upd[j] = run[j];
-        if (!group_barrier(meet[0], nch, st)) return;
+        if (!group_barrier<CL>(meet[0], nch, st)) return;
 
         // ---- B: s = (m^2 + sigma_0) p - D_eo h on the even site k, Re<p, s>
         vec3<R> s[NR];
@@ -556,7 +595,7 @@ __global__ void __launch_bounds__(MS_SMALL_BLOCK, MINB) ms_small_kernel(MSSmallA
             }
         }
         double tot[NR];
-        if (!group_exchange<NR, false>(red, tot, meet[1], nch, chunk, st)) return;
+        if (!group_exchange<NR, false, CL>(red, tot, meet[1], nch, chunk, st)) return;
 
         // ---- C: omega, the shifted recurrences (FinAlpha), r += omega s, |r|^2
 #pragma unroll
@@ -598,7 +637,7 @@ __global__ void __launch_bounds__(MS_SMALL_BLOCK, MINB) ms_small_kernel(MSSmallA
                 stcg3<R>(a.ring + ((size_t)wp * a.nrhs + r0 + j) * stride, Vh, k, r[j]);
             }
         }
-        if (!group_exchange<NR, true>(red, tot, meet[2], nch, chunk, st)) return;
+        if (!group_exchange<NR, true, CL>(red, tot, meet[2], nch, chunk, st)) return;
 
         // ---- gamma, freezing (FinLambda)
 #pragma unroll
