@@ -62,8 +62,23 @@ struct DslashArgs {
     const int *stop;    // optional: skip the launch when *stop != 0 ...
     int *stop_set;      // ... and then set *stop_set = 1 (solver loop control)
     const int *run_if;  // optional: skip the launch when *run_if == 0
+    int down;           // 1: walk the tiles from the last to the first (walk_alternates)
     int k_lo, k_count;  // output sites [k_lo, k_lo + k_count) (k_count 0: all Vh); no RED with a range
 };
+
+// Whether launches of NR right-hand sides with links LF should walk the sites in alternating
+// directions (odd outputs upwards, even ones downwards, the solvers' vector kernels likewise), so
+// that each starts on what the one before it left in L2.  M^dag M, FP64, against one direction:
+// 24x20^2x18 1.15-1.24 times as fast with 18-real links and 2 or 4 right-hand sides, 24^3x32 1.05.
+// Where links and vectors stay in L2 between launches it only moves them between the two dies'
+// halves: 20^2x16x18 two right-hand sides (83 MB) 0.87, 18x14x16x22 eight (85 MB) 0.94, at 99 to
+// 110 MB neither, from 116 MB faster (L2: 126 MB).
+template <class LF, int NR>
+inline bool walk_alternates(long Vh)
+{
+    const double bytes = (double)Vh * (8.0 * LF::bytes + 3.0 * NR * LF::store::planes * sizeof(typename LF::store::elem) / LF::store::pack);
+    return bytes > 105e6;
+}
 
 // Re<y, o> of one colour added to a site's term of the fused reduction: FP64 products for FP64
 // spinors; for FP32 spinors the site term is summed in FP32 with fixed rounding and converted to
@@ -95,11 +110,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) dslash_kernel(DslashArgs<LF, NR, 
     typedef typename S::elem E;
     // tiles of BLOCK consecutive output sites; a launch with fewer blocks than tiles (persistent
     // blocks) walks them with stride gridDim.x, so the per-block work of the fused reduction
-    // (fence, ticket) is paid once per block instead of once per tile.  Launches onto the even sites
-    // walk the tiles downwards and those onto the odd sites upwards (and the solvers' vector kernels
-    // alternate likewise), so a launch starts on what the one before it left in L2.
+    // (fence, ticket) is paid once per block instead of once per tile
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const int tile = a.p_out == 0 ? ntiles - 1 - t : t;
+        const int tile = a.down ? ntiles - 1 - t : t;
         const int k = a.k_lo + tile * BLOCK + threadIdx.x;
         if constexpr (S::pack > 1) {
             // packed right-hand sides: one load brings P of them (PackS)

@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(VEC_BLOCK) ms_resid_kernel(int Vh, size_t stri
 // p = r_m + gamma p (the base search direction; the shifted p_i and x_i are updated once per
 // window by ms_flush_kernel)
 template <typename Rv, int NR>
-__global__ void __launch_bounds__(VEC_BLOCK) ms_update_kernel(int Vh, size_t stride, const typename MSVec<Rv>::E *__restrict__ ring,
+__global__ void __launch_bounds__(VEC_BLOCK) ms_update_kernel(int Vh, size_t stride, int down, const typename MSVec<Rv>::E *__restrict__ ring,
                                                                typename MSVec<Rv>::E *p, MSState *st)
 {
     typedef typename MSVec<Rv>::E E;
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(VEC_BLOCK) ms_update_kernel(int Vh, size_t str
     typedef PackIO<Rv, P> IO;
     typedef PackElem<Rv, P> PE;
     if (*(volatile int *)&st->stop_k4) return;
-    const int k = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;  // downwards, K3 went upwards
+    const int k = (down ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * blockDim.x + threadIdx.x;  // K3 went upwards
     if (k >= Vh) return;
     const E *r = ring + (size_t)(*(volatile const int *)&st->wpos - 1) * NR * stride;  // K3 advanced wpos
 #pragma unroll

@@ -226,12 +226,12 @@ __global__ void __launch_bounds__(VEC_BLOCK) rb_xr_kernel(int Vh, size_t stride,
 
 // p = rs + beta p
 template <int NR, class S>
-__global__ void __launch_bounds__(VEC_BLOCK) rb_p_kernel(int Vh, size_t sstride, const typename S::elem *__restrict__ rs,
+__global__ void __launch_bounds__(VEC_BLOCK) rb_p_kernel(int Vh, size_t sstride, int down, const typename S::elem *__restrict__ rs,
                                                           typename S::elem *p, const RBState *st)
 {
     typedef typename S::real Rs;
     if (*(volatile const int *)&st->stop) return;
-    const int k = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;  // downwards, rb_xr_kernel went upwards
+    const int k = (down ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * blockDim.x + threadIdx.x;  // rb_xr_kernel went upwards
     if (k >= Vh) return;
 #pragma unroll
     for (int j = 0; j < NR; j++) {
@@ -318,6 +318,8 @@ static int rb_group(rhmc_ctx *c, const LF &lf, const double *coef, const double 
     s2.stride = sstride; s2.beta = (Rs)-0.5; s2.use_alphas = 1;
     for (int j = 0; j < NR; j++) s2.alphas[j] = (Rs)coef[j];
     s2.partials = pt; s2.ticket = tk + 1; s2.fin.st = st; s2.stop = &st->stop;
+    const int down = walk_alternates<LF, NR>(Vh);
+    s2.down = down;
 
     struct Key {
         int kind, link_reals, link_bytes, nr, n_ru, vh;
@@ -352,7 +354,7 @@ static int rb_group(rhmc_ctx *c, const LF &lf, const double *coef, const double 
             dslash_launch_cand<LF, NR, true, true, FinRBAlpha<NR>>(key.cand[2], s2, Vh, s_);
             rb_xr_kernel<NR, S, X><<<persistent_grid((const void *)rb_xr_kernel<NR, S, X>, VEC_BLOCK, gv), VEC_BLOCK, 0,
                                      s_>>>(Vh, stride, sstride, (X *)xs, (E *)rs, (const E *)p, (const E *)ap, pt, tk + 2, st);
-            rb_p_kernel<NR, S><<<gv, VEC_BLOCK, 0, s_>>>(Vh, sstride, (const E *)rs, (E *)p, st);
+            rb_p_kernel<NR, S><<<gv, VEC_BLOCK, 0, s_>>>(Vh, sstride, down, (const E *)rs, (E *)p, st);
         }
         ce = cudaStreamEndCapture(s_, &graph);
         if (ce != cudaSuccess) return cuda_fail(ce, "refine capture");
