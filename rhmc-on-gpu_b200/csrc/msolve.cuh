@@ -29,6 +29,7 @@
 #include <cstddef>
 
 #include "dslash.cuh"
+#include "solver.h"
 
 namespace rhmc {
 
@@ -384,7 +385,7 @@ __global__ void __launch_bounds__(VEC_BLOCK) ms_resid_kernel(int Vh, size_t stri
     typedef typename MSVec<Rv>::E E;
     if (*(volatile int *)&st->stop) return;
     const int wp = *(volatile const int *)&st->wpos;
-    const E *rprev = ring + (size_t)(wp == 0 ? win - 1 : wp - 1) * NR * stride;
+    const E *rprev = ring + (size_t)ms_prev_slot(wp, win) * NR * stride;
     E *r = ring + (size_t)wp * NR * stride;
     int run[NR];
     Rv om[NR];
@@ -445,7 +446,7 @@ __global__ void __launch_bounds__(VEC_BLOCK) ms_resid_kernel(int Vh, size_t stri
 // p = r_m + gamma p (the base search direction; the shifted p_i and x_i are updated once per
 // window by ms_flush_kernel)
 template <typename Rv, int NR>
-__global__ void __launch_bounds__(VEC_BLOCK) ms_update_kernel(int Vh, size_t stride, int down, const typename MSVec<Rv>::E *__restrict__ ring,
+__global__ void __launch_bounds__(VEC_BLOCK) ms_update_kernel(int Vh, size_t stride, int win, int down, const typename MSVec<Rv>::E *__restrict__ ring,
                                                                typename MSVec<Rv>::E *p, MSState *st)
 {
     typedef typename MSVec<Rv>::E E;
@@ -455,7 +456,9 @@ __global__ void __launch_bounds__(VEC_BLOCK) ms_update_kernel(int Vh, size_t str
     if (*(volatile int *)&st->stop_k4) return;
     const int k = (down ? gridDim.x - 1 - blockIdx.x : blockIdx.x) * blockDim.x + threadIdx.x;  // K3 went upwards
     if (k >= Vh) return;
-    const E *r = ring + (size_t)(*(volatile const int *)&st->wpos - 1) * NR * stride;  // K3 advanced wpos
+    // K3 advanced wpos, unless K2 met a non-finite or zero <p,s> and stopped the solve before it: then
+    // wpos may still be 0 (the other right-hand sides' p is formed once more and not used)
+    const E *r = ring + (size_t)ms_prev_slot(*(volatile const int *)&st->wpos, win) * NR * stride;
 #pragma unroll
     for (int q = 0; q < NR / P; q++) {
         int run[P], any = 0;

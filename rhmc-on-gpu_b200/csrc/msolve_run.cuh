@@ -234,7 +234,7 @@ static int ms_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *
             dslash_launch_cand<LFB, NR, true, true, FinAlpha<NR>>(key.cand[1], a2, Vh, s_);
             ms_resid_kernel<Rv, NR><<<persistent_grid((const void *)ms_resid_kernel<Rv, NR>, VEC_BLOCK, gv), VEC_BLOCK, 0,
                                       s_>>>(Vh, stride, win, (E *)r, (const E *)s, pt, tk + 2, st);
-            ms_update_kernel<Rv, NR><<<gv, VEC_BLOCK, 0, s_>>>(Vh, stride, down, (const E *)r, (E *)p, st);
+            ms_update_kernel<Rv, NR><<<gv, VEC_BLOCK, 0, s_>>>(Vh, stride, win, down, (const E *)r, (E *)p, st);
         }
         ms_flush_kernel<Rv, NR><<<grid_for((long)Vh * BasePack<Rv, NR>::P, VEC_BLOCK), VEC_BLOCK, coef_bytes, s_>>>(
             Vh, S, stride, (const E *)r, (double2 *)ps, xs, tk + 3, st);

@@ -6,6 +6,10 @@ struct rhmc_ctx;
 
 namespace rhmc {
 
+// Slot of a window's residual ring before slot m (0 <= m <= win): the window's first iteration continues
+// from the last slot.
+__host__ __device__ inline int ms_prev_slot(int m, int win) { return m == 0 ? win - 1 : m - 1; }
+
 struct MSolveArgs {
     int nshift, nrhs;
     const double *shift;  // absolute shifts sigma_{r,i}, [nrhs][nshift] (each RHS its own pole set)

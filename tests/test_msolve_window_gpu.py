@@ -87,3 +87,20 @@ def test_short_window_when_memory_is_short(torch_cuda):
         ctx.close()
     assert held[0] - held[1] == 8 * nrhs * spinor  # the ring: 16 or 8 slots
     assert float((out[0] - out[1]).norm() / out[0].norm()) < 1e-13
+
+
+def test_zero_product_in_the_first_iteration(torch_cuda):
+    """A right-hand side that is zero in FP32 but not in FP64 gives <p,s> = 0 in the very first iteration:
+    the batch ends with the non-finite error, and the context solves on as if it had not happened."""
+    dims = (24, 16, 16, 16)  # too large for one kernel
+    ctx = G.new_ctx(dims, mass=0.3)
+    ctx.set_gauge(F.random_links(dims, seed=31, kind="near1"))
+    src = F.random_spinor(dims, seed=32, n=4)
+    b = G.to_internal(ctx, rb.LINKS_F64_18, src)
+    args = (4, rb.MSOLVE_FP32, rb.LINKS_F32_12, 1e-3)
+    want, _ = _solve(ctx, b, *args)
+    src[1] *= 1e-60
+    with pytest.raises(rb.RhmcError, match="non-finite"):
+        _solve(ctx, G.to_internal(ctx, rb.LINKS_F64_18, src), *args)
+    again, _ = _solve(ctx, b, *args)
+    assert torch_cuda.equal(want, again)
