@@ -505,6 +505,7 @@ __global__ void __launch_bounds__(VEC_BLOCK, 2) ms_flush_kernel(int Vh, int nshi
 {
     extern __shared__ double2 s_coef[];  // [rhs][nshift][MS_WIN + 1] (cx, cb), entry MS_WIN (cx0, ca)
     __shared__ int s_list[NR][MS_MAX_SHIFT], s_n[NR];  // active shifts, 2 i + (p_i is needed further)
+    __shared__ unsigned s_wrote[NR];                   // the window's iterations of a right-hand side, a bit each
     static_assert(NR <= VEC_BLOCK / 32 && MS_MAX_SHIFT <= 32, "a warp per right-hand side, a lane per shift");
     constexpr int P = BasePack<Rv, NR>::P;
     const int rstride = nshift * (MS_WIN + 1) + 1;  // one element of padding: other banks for another RHS
@@ -512,7 +513,8 @@ __global__ void __launch_bounds__(VEC_BLOCK, 2) ms_flush_kernel(int Vh, int nshi
     {
         const int j = threadIdx.x >> 5, i = threadIdx.x & 31;
         if (j < NR) {
-            int any = 0, an = 0;
+            int an = 0;
+            unsigned took = 0;  // iterations that updated the shift
             if (i < nshift) {
                 const MSHist &hq = st->hist[j];
                 double2 *cf = s_coef + (size_t)j * rstride + i * (MS_WIN + 1);
@@ -539,7 +541,7 @@ __global__ void __launch_bounds__(VEC_BLOCK, 2) ms_flush_kernel(int Vh, int nshi
                         if (act[m]) {
                             D = om[m] + ga[m] * D;
                             G = ga[m] * G;
-                            any = 1;
+                            took |= 1u << (m0 + m);
                         }
                     }
                 }
@@ -548,8 +550,9 @@ __global__ void __launch_bounds__(VEC_BLOCK, 2) ms_flush_kernel(int Vh, int nshi
             // p_i is written for every shift still active, also when the RHS stopped in this window:
             // a later phase may resume it from exactly this state.  The first window visits every
             // shift: x_i is in memory only after it.
-            const int use = i < nshift && (any || first);
-            const unsigned mask = __ballot_sync(0xffffffffu, use);
+            const int use = i < nshift && (took || first);
+            const unsigned mask = __ballot_sync(0xffffffffu, use), wrote = __reduce_or_sync(0xffffffffu, took);
+            if (i == 0) s_wrote[j] = wrote;
             if (use) s_list[j][__popc(mask & ((1u << i) - 1u))] = 2 * i + (an ? 1 : 0);
             if (i == 0) s_n[j] = __popc(mask);
         }
@@ -560,16 +563,19 @@ __global__ void __launch_bounds__(VEC_BLOCK, 2) ms_flush_kernel(int Vh, int nshi
     if (k < Vh && (wp > 0 || first)) {
         for (int q = 0; q < NR / P; q++) {
             const int j = q * P + l, n = s_n[j];
+            const unsigned wrote = s_wrote[j];
             if (n == 0) continue;
             const double2 *cj = s_coef + (size_t)j * rstride;
 #pragma unroll 1
             for (int c = 0; c < 3; c++) {
                 const size_t o = (size_t)j * nshift * stride + (size_t)c * Vh + k;
-                double2 rv[MS_WIN];  // slots past wp hold older residuals and have zero coefficients
+                // only slots that this right-hand side wrote in this window: the others (it was zero, or had
+                // stopped) have zero coefficients but may hold anything, also NaN from memory or an older solve
+                double2 rv[MS_WIN];
 #pragma unroll
                 for (int m = 0; m < MS_WIN; m++) {
                     rv[m] = make_double2(0.0, 0.0);
-                    if (m < wp) {
+                    if (wrote >> m & 1u) {
                         const typename MSVec<Rv>::E e = __ldg(ring + (size_t)m * NR * stride + bidx<Rv, NR>(j, c, k, Vh));
                         rv[m] = make_double2((double)e.x, (double)e.y);
                     }

@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(MS_SMALL_BLOCK, MINB) ms_small_kernel(MSSmallA
 #pragma unroll
                     for (int m = 0; m < MS_WIN; m++) {
                         rv[m] = make_double2(0.0, 0.0);
-                        if (m < wp) {
+                        if (m < wp && s_act[j][m]) {  // a slot this right-hand side wrote (see ms_flush_kernel)
                             const E e = __ldcg(a.ring + ((size_t)m * a.nrhs + r0 + j) * stride + (size_t)c * Vh + k);
                             rv[m] = make_double2((double)e.x, (double)e.y);
                         }

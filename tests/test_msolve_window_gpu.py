@@ -104,3 +104,38 @@ def test_zero_product_in_the_first_iteration(torch_cuda):
         _solve(ctx, G.to_internal(ctx, rb.LINKS_F64_18, src), *args)
     again, _ = _solve(ctx, b, *args)
     assert torch_cuda.equal(want, again)
+
+
+# two right-hand sides a block (256 chunks), launched FP64, launched FP32 in packs of four
+@pytest.mark.parametrize("dims,nrhs,mode,fmt,res", [((16, 16, 16, 16), 2, rb.MSOLVE_FP64, rb.LINKS_F64_18, 1e-8),
+                                                    ((16, 16, 16, 16), 4, rb.MSOLVE_FP64, rb.LINKS_F64_12, 1e-8),
+                                                    ((24, 16, 16, 16), 4, rb.MSOLVE_FP32, rb.LINKS_F32_12, 1e-4)])
+@pytest.mark.parametrize("scale", [0.0, 1e-12])
+def test_slots_a_right_hand_side_did_not_write(torch_cuda, dims, nrhs, mode, fmt, res, scale):
+    """A right-hand side that is zero (scale 0) or stops after one iteration, beside others that go on, over a
+    ring that holds NaN in a later slot of it: its solutions are those of a solve in a new context."""
+    if scale and mode == rb.MSOLVE_FP32:
+        scale = 1e-8
+    src = F.random_spinor(dims, seed=42, n=nrhs)
+    src[-1] *= scale
+    links = F.random_links(dims, seed=41, kind="near1")
+    out = []
+    for poison in (False, True):
+        ctx = G.new_ctx(dims, mass=0.3)
+        ctx.set_gauge(links)
+        b = G.to_internal(ctx, rb.LINKS_F64_18, src)
+        x, info = _solve(ctx, b, nrhs, mode, fmt, res)
+        if poison:
+            # the initial residual of a single solve lies in slot 15, which in the ring of nrhs right-hand
+            # sides is slot 15 // nrhs of number 15 % nrhs = nrhs - 1
+            bad = torch_cuda.full((6 * ctx.Vh,), float("nan"), dtype=torch_cuda.float64, device="cuda")
+            with pytest.raises(rb.RhmcError, match="non-finite"):
+                _solve(ctx, bad, 1, mode, fmt, res)
+            x, info = _solve(ctx, b, nrhs, mode, fmt, res)
+        assert info["status"] == 0 and info["iters"][nrhs - 1] == (1 if scale else 0) and info["iters"][0] > 8
+        out.append(x)
+        ctx.close()
+    assert torch_cuda.isfinite(out[0]).all()
+    assert torch_cuda.equal(out[0], out[1])
+    if not scale:
+        assert (out[1][-out[1].numel() // nrhs:] == 0).all()
