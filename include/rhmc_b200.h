@@ -155,8 +155,7 @@ typedef struct {
                               1e-3 |b| but no more than 1e7 x `residual` above the target (the FP32
                               part leaves the shifted systems near 1e-7 of the hand-over residual)
                               and no less than 1e-4 |b| */
-    double ru_delta;       /* mixed mode: FP32 residual reduction between FP64 updates (0: 0.05); a system
-                              is also updated once its sloppy residual is a tenth of `residual` */
+    double ru_delta;       /* mixed mode: FP32 residual reduction between FP64 updates (0: 0.05) */
     int certify;           /* FP64 mode: afterwards refine, by FP64 CG one system at a time, every system
                               whose FP64 true residual is still above `residual` (the reference's
                               iterated-residual test alone can stop above it) */
