@@ -26,7 +26,10 @@ struct Workspace {
         if (it != buf.end()) { cudaFree(it->second.first); buf.erase(it); }
         void *p = nullptr;
         cudaError_t e = cudaMalloc(&p, bytes ? bytes : 16);
-        if (e != cudaSuccess) return e;
+        if (e != cudaSuccess) {
+            cudaGetLastError();  // the caller reports it; later launches start clean
+            return e;
+        }
         buf[name] = std::make_pair(p, bytes);
         *out = p;
         return cudaSuccess;

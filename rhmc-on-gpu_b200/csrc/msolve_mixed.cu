@@ -160,17 +160,17 @@ int msolve_mixed(rhmc_ctx *c, int fmt, int nshift, const double *shifts, int nrh
     // refinement: half links and spinors for F16_12, else FP32 sloppy links of the matching width
     if (fmt == RHMC_LINKS_F16_12) {
         L16_12 lf;
-        links_f16_12(c, &lf);
+        CK(links_f16_12(c, &lf));
         rc = refine_all(c, lf, nshift, shifts, nrhs, res, max_iter, x, b, &it_b, &ru, ru_delta, RB_MAX,
                         tr.empty() ? nullptr : tr.data(), &nsys);
     } else if (fmt == RHMC_LINKS_F32_18 || fmt == RHMC_LINKS_F64_18) {
         L32_18 lf;
-        links_f32_18(c, &lf);
+        CK(links_f32_18(c, &lf));
         rc = refine_all(c, lf, nshift, shifts, nrhs, res, max_iter, x, b, &it_b, &ru, ru_delta, RB_MAX,
                         tr.empty() ? nullptr : tr.data(), &nsys);
     } else {
         L32_12 lf;
-        links_f32_12(c, &lf);
+        CK(links_f32_12(c, &lf));
         rc = refine_all(c, lf, nshift, shifts, nrhs, res, max_iter, x, b, &it_b, &ru, ru_delta, RB_MAX,
                         tr.empty() ? nullptr : tr.data(), &nsys);
     }
@@ -246,7 +246,7 @@ static int msolve_fp64(rhmc_ctx *c, const rhmc_msolve_params *P, const double *s
         for (double &v : tr) v = std::sqrt(v);
         if (rc == RHMC_OK) {
             L64_18 lf;
-            links_f64_18(c, &lf);
+            CK(links_f64_18(c, &lf));
             rc = refine_all(c, lf, P->nshift, sh, P->nrhs, P->residual, P->max_iter, x, b, &it_b, &ru, 0.05, 1, tr.data(), &nsys);
         }
         cudaStreamSynchronize(c->stream);

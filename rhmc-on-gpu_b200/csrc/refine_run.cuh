@@ -270,7 +270,7 @@ static int rb_group(rhmc_ctx *c, const LF &lf, const double *coef, const double 
     CK(c->ws.get("rb_partials", (size_t)red_chunks(Vh) * 2 * NR * sizeof(double), &part));
     CK(c->ws.get("rb_tickets", 4 * sizeof(unsigned), &tick));
     L64_18 l64;
-    links_f64_18(c, &l64);
+    CK(links_f64_18(c, &l64));
     RBState *st = (RBState *)stv;
     unsigned *tk = (unsigned *)tick;
     double *pt = (double *)part;
