@@ -186,7 +186,13 @@ typedef struct {
  * (the ShiftMultiFermion order [no_ps][order][sizeh], lib/Action/fermions.h:114).
  * Returns RHMC_ERR_MAXITER instead of the reference's exit(1) at max_cg. */
 int rhmc_msolve(rhmc_ctx *ctx, const rhmc_msolve_params *p, double *x, const double *b, rhmc_msolve_info *info);
-/* Same with host arrays in the reference layout: b complex[nrhs][Vh][3], x complex[nrhs][nshift][Vh][3]. */
+/* Iterations per window of the last multi-shift phase (0 before the first): a solve applies the updates of
+ * its shifted vectors together once per window, 16 iterations, or 8 where the residuals of 16 would not
+ * leave the device the memory that the rest of the solve needs.  The solutions of the two differ by
+ * rounding.  The choice is made when the residuals' buffer has to grow and stands until it grows again or
+ * is released.  No counterpart in the reference. */
+int rhmc_msolve_window(const rhmc_ctx *ctx, int *iterations);
+/* rhmc_msolve with host arrays in the reference layout: b complex[nrhs][Vh][3], x complex[nrhs][nshift][Vh][3]. */
 int rhmc_msolve_host(rhmc_ctx *ctx, const rhmc_msolve_params *p, double *x, const double *b, rhmc_msolve_info *info);
 /* |b_r - (M^dag M + sigma_i) x_{r,i}| in FP64 for every (r, i); out: host double[nrhs][nshift].
  * The check of inverter.cc:306-338 / cu_inverter.cc:79-120 without the debug build. */

@@ -17,28 +17,66 @@ namespace rhmc {
 
 struct Driver;
 
+// Named scratch buffers.  The multi-shift solver's residual rings ("ms_r...") hold nothing between solves:
+// outside one they are given up when the device has no room for something else.
 struct Workspace {
     std::map<std::string, std::pair<void *, size_t>> buf;
+    bool in_solve = false;       // the rings are in use
+    bool out_of_memory = false;  // an allocation failed (reset at the start of a solve)
+    cudaError_t alloc(void **out, size_t bytes)
+    {
+        cudaError_t e = cudaMalloc(out, bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();  // the caller reports it; later launches start clean
+            if (!in_solve && drop_rings()) e = cudaMalloc(out, bytes);
+        }
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            *out = nullptr;
+            out_of_memory = out_of_memory || e == cudaErrorMemoryAllocation;
+        }
+        return e;
+    }
     cudaError_t get(const std::string &name, size_t bytes, void **out)
     {
         auto it = buf.find(name);
         if (it != buf.end() && it->second.second >= bytes) { *out = it->second.first; return cudaSuccess; }
         if (it != buf.end()) { cudaFree(it->second.first); buf.erase(it); }
         void *p = nullptr;
-        cudaError_t e = cudaMalloc(&p, bytes ? bytes : 16);
-        if (e != cudaSuccess) {
-            cudaGetLastError();  // the caller reports it; later launches start clean
-            return e;
-        }
+        cudaError_t e = alloc(&p, bytes ? bytes : 16);
+        if (e != cudaSuccess) return e;
         buf[name] = std::make_pair(p, bytes);
         *out = p;
         return cudaSuccess;
+    }
+    size_t held(const std::string &name) const
+    {
+        const auto it = buf.find(name);
+        return it == buf.end() ? 0 : it->second.second;
+    }
+    bool drop_rings()
+    {
+        bool any = false;
+        for (auto it = buf.lower_bound("ms_r"); it != buf.end() && it->first.compare(0, 4, "ms_r") == 0;) {
+            cudaFree(it->second.first);
+            it = buf.erase(it);
+            any = true;
+        }
+        return any;
     }
     void release()
     {
         for (auto &kv : buf) cudaFree(kv.second.first);
         buf.clear();
     }
+};
+
+// Iterations per window of the multi-shift solves (ms_ring).
+struct WindowChoice {
+    std::map<std::string, bool> short_ring;  // rings that were made for half windows
+    bool half_only = false;                  // a solve repeated because the device ran out of memory
+    bool was_long = false;                   // some phase of the present call ran whole windows
+    int last = 0;                            // iterations per window of the last phase
 };
 
 // Instantiated CUDA graphs of the solver loops, keyed by everything their kernels capture
@@ -107,6 +145,7 @@ struct rhmc_ctx {
     double *P;
     double *IP;
     rhmc::Workspace ws;
+    rhmc::WindowChoice window;
     int *hflags;   // pinned host words for polling device-side solver flags
     // graph-captured solver loops run on this stream, ordered against `stream` by events
     // (capture is not possible on the legacy default stream a caller may have installed)

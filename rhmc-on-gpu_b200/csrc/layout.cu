@@ -266,14 +266,11 @@ static cudaError_t ensure_derived(rhmc_ctx *c, int fmt)
     void *p = nullptr;
     cudaError_t e = cudaSuccess;
     const size_t Vh = c->Vh;
-    if (fmt == RHMC_LINKS_F64_12 && !c->U64_12) e = cudaMalloc(&p, 8 * 6 * Vh * sizeof(double2)), c->U64_12 = (double2 *)p;
-    if (fmt == RHMC_LINKS_F32_18 && !c->U32_18) e = cudaMalloc(&p, 8 * 4 * Vh * sizeof(float4) + 8 * Vh * sizeof(float2)), c->U32_18 = (float4 *)p;
-    if (fmt == RHMC_LINKS_F32_12 && !c->U32_12) e = cudaMalloc(&p, 8 * 3 * Vh * sizeof(float4)), c->U32_12 = (float4 *)p;
-    if (fmt == RHMC_LINKS_F16_12 && !c->U16_12) e = cudaMalloc(&p, 8 * Vh * (sizeof(uint4) + sizeof(uint2))), c->U16_12 = (uint4 *)p;
-    if (e != cudaSuccess) {
-        cudaGetLastError();  // the caller reports it; later launches start clean
-        return e;
-    }
+    if (fmt == RHMC_LINKS_F64_12 && !c->U64_12) e = c->ws.alloc(&p, 8 * 6 * Vh * sizeof(double2)), c->U64_12 = (double2 *)p;
+    if (fmt == RHMC_LINKS_F32_18 && !c->U32_18) e = c->ws.alloc(&p, 8 * 4 * Vh * sizeof(float4) + 8 * Vh * sizeof(float2)), c->U32_18 = (float4 *)p;
+    if (fmt == RHMC_LINKS_F32_12 && !c->U32_12) e = c->ws.alloc(&p, 8 * 3 * Vh * sizeof(float4)), c->U32_12 = (float4 *)p;
+    if (fmt == RHMC_LINKS_F16_12 && !c->U16_12) e = c->ws.alloc(&p, 8 * Vh * (sizeof(uint4) + sizeof(uint2))), c->U16_12 = (uint4 *)p;
+    if (e != cudaSuccess) return e;
     derive_links_kernel<<<grid_for(8L * c->Vh, 256), 256, 0, c->stream>>>(
         c->g, c->U64, fmt == RHMC_LINKS_F64_12 ? c->U64_12 : nullptr, fmt == RHMC_LINKS_F32_18 ? c->U32_18 : nullptr,
         fmt == RHMC_LINKS_F32_12 ? c->U32_12 : nullptr, fmt == RHMC_LINKS_F16_12 ? c->U16_12 : nullptr);

@@ -303,11 +303,8 @@ static int msolve_fp32(rhmc_ctx *c, const rhmc_msolve_params *P, const double *s
     return rc;
 }
 
-extern "C" {
-
-int rhmc_msolve(rhmc_ctx *c, const rhmc_msolve_params *P, double *x, const double *b, rhmc_msolve_info *info)
+static int msolve_any(rhmc_ctx *c, const rhmc_msolve_params *P, double *x, const double *b, rhmc_msolve_info *info)
 {
-    if (!c || !P || !x || !b || (!P->shifts && !P->rhs_shifts)) return fail(RHMC_ERR_ARG, "null argument");
     if (P->nshift < 1 || P->nshift > MS_MAX_SHIFT) return fail(RHMC_ERR_ARG, "nshift must be in [1, %d]", MS_MAX_SHIFT);
     if (P->nrhs < 1) return fail(RHMC_ERR_ARG, "nrhs must be >= 1");
     if (P->max_iter < 1) return fail(RHMC_ERR_ARG, "max_iter must be >= 1");
@@ -359,6 +356,38 @@ int rhmc_msolve(rhmc_ctx *c, const rhmc_msolve_params *P, double *x, const doubl
         return rc;
     }
     return fail(RHMC_ERR_ARG, "bad solver mode %d", P->mode);
+}
+
+extern "C" {
+
+int rhmc_msolve(rhmc_ctx *c, const rhmc_msolve_params *P, double *x, const double *b, rhmc_msolve_info *info)
+{
+    if (!c || !P || !x || !b || (!P->shifts && !P->rhs_shifts)) return fail(RHMC_ERR_ARG, "null argument");
+    c->ws.in_solve = true;
+    c->ws.out_of_memory = false;
+    c->window.was_long = false;
+    int rc = msolve_any(c, P, x, b, info);
+    if (rc == RHMC_ERR_CUDA && c->ws.out_of_memory && c->window.was_long) {
+        // Out of memory beside a ring of whole windows: once more with half ones, whose ring is half as
+        // long, unless x overlaps b, which then is not what it was.
+        const double *xe = x + (size_t)P->nrhs * P->nshift * 6 * c->Vh, *be = b + (size_t)P->nrhs * 6 * c->Vh;
+        cudaStreamSynchronize(c->stream);
+        c->ws.drop_rings();
+        if (xe <= b || be <= x) {
+            c->window.half_only = true;
+            rc = msolve_any(c, P, x, b, info);
+            c->window.half_only = false;
+        }
+    }
+    c->ws.in_solve = false;
+    return rc;
+}
+
+int rhmc_msolve_window(const rhmc_ctx *c, int *iterations)
+{
+    if (!c || !iterations) return fail(RHMC_ERR_ARG, "null argument");
+    *iterations = c->window.last;
+    return RHMC_OK;
 }
 
 int rhmc_msolve_host(rhmc_ctx *c, const rhmc_msolve_params *P, double *x, const double *b, rhmc_msolve_info *info)

@@ -66,20 +66,39 @@ static inline int ms_result(const MSState &hs, const MSolveArgs &A, MSolveInfo *
 }
 
 // The residual ring of a phase, `slot` bytes per iteration, and the iterations per window it allows:
-// MS_WIN when the ring is already that long, small (the query of free memory costs a new context's
-// first solve a millisecond or more) or fits with room to spare for what the rest of a solve may
-// still allocate (true residuals 16, refinement at most 52 FP64 spinors of v64 bytes), else half.
-static inline cudaError_t ms_ring(rhmc_ctx *c, const std::string &name, size_t slot, size_t v64, void **ring, int *win)
+// MS_WIN where the ring is already that long or the device has room for it and for what the rest of a
+// solve may still allocate (`later` FP64 spinors of v64 bytes), else half.  Only a ring that must grow asks
+// for the free memory, and not when all of it is small (the query costs a new context's first solve a
+// millisecond or more); a choice against the longer ring stands until the ring has to grow again.
+// Where the estimate proves too low the solve is repeated with half windows (rhmc_msolve).
+static inline cudaError_t ms_ring(rhmc_ctx *c, const std::string &name, size_t slot, size_t v64, int later, void **ring, int *win)
 {
-    const auto it = c->ws.buf.find(name);
-    const size_t have = it == c->ws.buf.end() ? 0 : it->second.second, want = MS_WIN * slot;
-    *win = MS_WIN;
-    if (have < want && want + 68 * v64 > ((size_t)1 << 28)) {
+    const size_t have = c->ws.held(name), want = MS_WIN * slot, rest = later * v64;
+    bool &half = c->window.short_ring[name];
+    bool whole = have >= want;
+    if (!whole && !(half && have >= want / 2) && !c->window.half_only) {
+        whole = true;
         size_t free_bytes = 0, total = 0;
-        if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || free_bytes + have < want + 68 * v64) *win = MS_WIN / 2;
+        if (want + rest > ((size_t)1 << 28))
+            whole = cudaMemGetInfo(&free_bytes, &total) == cudaSuccess && free_bytes + have >= want + rest;
     }
-    return c->ws.get(name, *win * slot, ring);
+    cudaError_t e = cudaSuccess;
+    if (whole) {
+        e = c->ws.get(name, want, ring);
+        whole = e != cudaErrorMemoryAllocation;
+    }
+    *win = c->window.last = whole ? MS_WIN : MS_WIN / 2;
+    half = !whole;
+    if (whole)
+        c->window.was_long = true;
+    else
+        e = c->ws.get(name, want / 2, ring);
+    return e;
 }
+
+// What a solve may allocate after a phase's ring, in FP64 spinors: true residuals 16, refinement 52, links
+// of the refinement 12, and where an FP32 phase follows (tau) its p, h, s and a short ring in FP32.
+static inline int ms_later(const MSolveArgs &A) { return 80 + (A.tau != 0.0 ? 6 * A.nrhs + 12 : 0); }
 
 // One phase of the multi-shift CG with links LF: base vectors (residual ring, p, h, s) in the
 // links' precision, shifted solutions and directions always FP64.  A fresh phase starts from
@@ -109,7 +128,7 @@ static int ms_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *
     CK(c->ws.get("ms_tickets", 8 * sizeof(unsigned), &tick));
     // ring of the window's residuals [slot][rhs]
     int win;
-    CK(ms_ring(c, vname("ms_r", sizeof(E)), NR * vbytes, v64, &r, &win));
+    CK(ms_ring(c, vname("ms_r", sizeof(E)), NR * vbytes, v64, ms_later(A), &r, &win));
     const int ru_every = (A.ru_every + win - 1) / win;  // in windows
     MSState *st = (MSState *)stv;
     unsigned *tk = (unsigned *)tick;
@@ -332,7 +351,7 @@ static int ms_small_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolve
     const size_t slot_bytes = (size_t)(n / NR) * 3 * ms_small_slots(NR, nch) * sizeof(ulonglong2);
     CK(c->ws.get("ms_slots", slot_bytes, &slots));
     int win;
-    CK(ms_ring(c, vname("ms_r", sizeof(E)), n * vbytes, v64, &r, &win));
+    CK(ms_ring(c, vname("ms_r", sizeof(E)), n * vbytes, v64, ms_later(A), &r, &win));
     MSState *st = (MSState *)stv;
 
     MSState hs;

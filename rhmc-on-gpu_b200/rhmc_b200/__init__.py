@@ -299,6 +299,13 @@ def _ctx_msolve_host(self, b, shifts, residual, max_iter=100000, mode=MSOLVE_FP6
     return (x[0] if single else x), info.as_dict()
 
 
+def _ctx_msolve_window(self):
+    """Iterations per window of the last multi-shift phase (16, or 8 where memory was short)."""
+    n = ctypes.c_int()
+    self.call("rhmc_msolve_window", ctypes.byref(n))
+    return n.value
+
+
 def _ctx_true_residuals(self, x, b, shifts, nrhs=1):
     sh = np.ascontiguousarray(shifts, np.float64)
     out = np.zeros((nrhs, len(sh)), np.float64)
@@ -308,6 +315,7 @@ def _ctx_true_residuals(self, x, b, shifts, nrhs=1):
 
 Context.msolve = _ctx_msolve
 Context.msolve_host = _ctx_msolve_host
+Context.msolve_window = _ctx_msolve_window
 Context.true_residuals = _ctx_true_residuals
 
 
