@@ -215,10 +215,13 @@ static int ms_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *
         for (int rr = 0; rr < NR; rr++) u2.alphas[rr] = c->mass * c->mass + A.base[rr];
     }
 
-    // shared memory of the flush's coefficients: above the 48 KB default for wide batches of many poles
-    const size_t coef_bytes = (size_t)NR * (S * (MS_WIN + 1) + 1) * sizeof(double2);
-    if (coef_bytes > 48 * 1024)
-        CK(cudaFuncSetAttribute(ms_flush_kernel<Rv, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)coef_bytes));
+    // shared memory of the flush's coefficients: above the 48 KB default for wide batches of many poles.
+    // The limit belongs to the process, so it is always that of the most poles: one of this call's size
+    // could be lowered by another context's call between here and the launch.
+    const auto coefs = [](int poles) { return (size_t)NR * (poles * (MS_WIN + 1) + 1) * sizeof(double2); };
+    const size_t coef_bytes = coefs(S);
+    if (coefs(MS_MAX_SHIFT) > 40 * 1024)
+        CK(cudaFuncSetAttribute(ms_flush_kernel<Rv, NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)coefs(MS_MAX_SHIFT)));
     const int chunk = win;  // one graph replay = one delayed-update window
     struct Key {
         int kind, link_reals, link_bytes, nr, chunk, nshift, vh, ru_every;

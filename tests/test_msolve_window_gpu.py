@@ -139,3 +139,36 @@ def test_slots_a_right_hand_side_did_not_write(torch_cuda, dims, nrhs, mode, fmt
     assert torch_cuda.equal(out[0], out[1])
     if not scale:
         assert (out[1][-out[1].numel() // nrhs:] == 0).all()
+
+
+def test_two_threads_with_different_pole_counts(torch_cuda):
+    """Eight right-hand sides with 24 and with 32 poles, both above the default limit of shared memory, in two
+    contexts and threads that each capture their solver graph anew."""
+    import threading
+    dims = (12, 12, 12, 12)
+    links = F.random_links(dims, seed=51, kind="near1")
+    src = F.random_spinor(dims, seed=52, n=8)
+    failed = []
+
+    def work(poles):
+        try:
+            ctx = G.new_ctx(dims, mass=0.5)
+            ctx.set_gauge(links)
+            b = G.to_internal(ctx, rb.LINKS_F64_18, src)
+            x = torch_cuda.empty(8 * poles * 6 * ctx.Vh, dtype=torch_cuda.float64, device="cuda")
+            torch_cuda.cuda.synchronize()
+            shifts = np.geomspace(0.1, 50.0, poles)
+            for _ in range(40):
+                info = ctx.msolve(x, b, shifts, 1e-6, nrhs=8, mode=rb.MSOLVE_FP64, fmt=rb.LINKS_F64_18)
+                assert info["status"] == 0
+                ctx.call("rhmc_workspace_release")
+            ctx.close()
+        except Exception as err:
+            failed.append(err)
+
+    threads = [threading.Thread(target=work, args=(n,)) for n in (24, 32)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
