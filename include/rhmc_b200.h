@@ -192,6 +192,11 @@ int rhmc_msolve(rhmc_ctx *ctx, const rhmc_msolve_params *p, double *x, const dou
  * rounding.  The choice is made when the residuals' buffer has to grow and stands until it grows again or
  * is released.  No counterpart in the reference. */
 int rhmc_msolve_window(const rhmc_ctx *ctx, int *iterations);
+/* enable = 0: solves of small lattices run launch by launch like those of large ones, instead of as one
+ * kernel whose blocks meet on the device (the default, 1, where the blocks fit).  Solutions and iteration
+ * counts are the same to the bit; for tests, and for a device on which the blocks cannot all be resident
+ * (the one-kernel solve then ends with RHMC_ERR_CUDA).  No counterpart in the reference. */
+int rhmc_msolve_one_kernel(rhmc_ctx *ctx, int enable);
 /* rhmc_msolve with host arrays in the reference layout: b complex[nrhs][Vh][3], x complex[nrhs][nshift][Vh][3]. */
 int rhmc_msolve_host(rhmc_ctx *ctx, const rhmc_msolve_params *p, double *x, const double *b, rhmc_msolve_info *info);
 /* |b_r - (M^dag M + sigma_i) x_{r,i}| in FP64 for every (r, i); out: host double[nrhs][nshift].

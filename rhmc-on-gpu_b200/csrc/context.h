@@ -146,6 +146,7 @@ struct rhmc_ctx {
     double *IP;
     rhmc::Workspace ws;
     rhmc::WindowChoice window;
+    bool one_kernel = true;  // small multi-shift solves may run as one kernel
     int *hflags;   // pinned host words for polling device-side solver flags
     // graph-captured solver loops run on this stream, ordered against `stream` by events
     // (capture is not possible on the legacy default stream a caller may have installed)

@@ -390,6 +390,13 @@ int rhmc_msolve_window(const rhmc_ctx *c, int *iterations)
     return RHMC_OK;
 }
 
+int rhmc_msolve_one_kernel(rhmc_ctx *c, int enable)
+{
+    if (!c) return fail(RHMC_ERR_ARG, "null context");
+    c->one_kernel = enable != 0;
+    return RHMC_OK;
+}
+
 int rhmc_msolve_host(rhmc_ctx *c, const rhmc_msolve_params *P, double *x, const double *b, rhmc_msolve_info *info)
 {
     if (!c || !P || !x || !b) return fail(RHMC_ERR_ARG, "null argument");

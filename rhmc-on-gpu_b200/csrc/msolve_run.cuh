@@ -433,7 +433,7 @@ template <class LF>
 int ms_run(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *info)
 {
     int rc = RHMC_OK;
-    if (A.fresh && A.ru_every == 0 && ms_small<LF>(c, lf, A, info, &rc)) return rc;
+    if (c->one_kernel && A.fresh && A.ru_every == 0 && ms_small<LF>(c, lf, A, info, &rc)) return rc;
     switch (A.nrhs) {
     case 1: return ms_phase<LF, 1>(c, lf, A, info);
     case 2: return ms_phase<LF, 2>(c, lf, A, info);

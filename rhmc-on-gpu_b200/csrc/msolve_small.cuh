@@ -20,8 +20,10 @@
 // sums, their order, the Dslash and every update round exactly as in the kernels of msolve.cuh: a
 // right-hand side's solution does not depend on which of the two paths solved it.
 //
-// Co-residency: launched cooperatively; an exchange gives up after MS_SPIN_LIMIT polls, flags
-// MSState::status = 3 and every block leaves.
+// Co-residency: a group of 2 to MS_CLUSTER chunks is a cluster, which the hardware places as a whole and
+// whose barrier needs no limit (no block leaves before the last meeting); larger groups are launched
+// cooperatively, and their exchanges give up after MS_SPIN_LIMIT polls, flag MSState::status = 3 and
+// every block leaves.
 #pragma once
 #include <cooperative_groups.h>
 

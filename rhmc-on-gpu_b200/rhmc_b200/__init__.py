@@ -306,6 +306,11 @@ def _ctx_msolve_window(self):
     return n.value
 
 
+def _ctx_msolve_one_kernel(self, enable):
+    """Whether small multi-shift solves may run as one kernel (the default)."""
+    self.call("rhmc_msolve_one_kernel", int(bool(enable)))
+
+
 def _ctx_true_residuals(self, x, b, shifts, nrhs=1):
     sh = np.ascontiguousarray(shifts, np.float64)
     out = np.zeros((nrhs, len(sh)), np.float64)
@@ -316,6 +321,7 @@ def _ctx_true_residuals(self, x, b, shifts, nrhs=1):
 Context.msolve = _ctx_msolve
 Context.msolve_host = _ctx_msolve_host
 Context.msolve_window = _ctx_msolve_window
+Context.msolve_one_kernel = _ctx_msolve_one_kernel
 Context.true_residuals = _ctx_true_residuals
 
 

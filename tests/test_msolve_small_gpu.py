@@ -1,7 +1,7 @@
 """The one-kernel multi-shift solve of small lattices: the same bits whichever way a right-hand side is
-solved (one kernel with one or two right-hand sides a block, or launch by launch in a wide batch),
-over one chunk of sites, several, the edge between the two ways blocks meet, ragged lattices and
-solves longer than one launch."""
+solved (one kernel with one or two right-hand sides a block, alone or in a batch, or launch by
+launch), over every way that its blocks meet and the edges between them, ragged lattices and solves
+longer than one launch."""
 import numpy as np
 import pytest
 
@@ -20,8 +20,32 @@ def _case(dims, mass, n, seed):
     return ctx, F.random_spinor(dims, seed=seed + 1, n=n)
 
 
-# Vh: 128 (one chunk, exactly), 192, 4096 (32 chunks), 4200 (33), 10368 (81; a batch of 8 is launched)
-# and 27720 (217 ragged chunks: three blocks per SM for two, launched for 8)
+# chunks of 128 sites: 1; 2 (ragged), 15 and 16, which meet as a cluster; 17 (ragged) and 32, by slots; 33
+# (ragged), 81 and 217 (ragged), by counted arrivals
+CHUNKS = [(4, 4, 4, 4), (6, 4, 4, 4), (8, 8, 6, 10), (8, 8, 8, 8), (6, 6, 10, 12), (8, 8, 8, 16), (10, 10, 6, 14), (12, 12, 12, 12),
+          (18, 14, 10, 22)]
+
+
+@pytest.mark.parametrize("dims", CHUNKS)
+@pytest.mark.parametrize("mode,fmt,res", [(rb.MSOLVE_FP64, rb.LINKS_F64_18, 1e-8), (rb.MSOLVE_FP64, rb.LINKS_F64_12, 1e-8),
+                                          (rb.MSOLVE_FP32, rb.LINKS_F32_18, 1e-4), (rb.MSOLVE_MIXED, rb.LINKS_F32_12, 1e-8)])
+def test_same_bits_launch_by_launch(torch_cuda, dims, mode, fmt, res):
+    """Against the launched kernels (mixed mode: its FP64 part, which an FP32 phase continues)."""
+    ctx, b = _case(dims, 0.2, 3, 21)
+    for n in (1, 2, 3):
+        launched = []
+        for one in (1, 0):
+            ctx.msolve_one_kernel(one)
+            before = ctx.launch_count()
+            x, info = ctx.msolve_host(b[:n], SHIFTS, res, mode=mode, fmt=fmt)
+            launched.append((ctx.launch_count() - before, x, info["iters"][:n]))
+        if n < 3 or dims != CHUNKS[-1]:  # three right-hand sides of 217 chunks do not fit as one kernel
+            assert launched[0][0] < launched[1][0]
+        assert launched[0][2] == launched[1][2]
+        assert np.array_equal(launched[0][1], launched[1][1]), (dims, n)
+
+
+# batches of one kernel beside each other, and for the last two lattices of 8 launched
 @pytest.mark.parametrize("dims", [(4, 4, 4, 4), (6, 4, 4, 4), (8, 8, 8, 16), (10, 10, 6, 14), (12, 12, 12, 12), (18, 14, 10, 22)])
 @pytest.mark.parametrize("mode,fmt,res", [(rb.MSOLVE_FP64, rb.LINKS_F64_18, 1e-8), (rb.MSOLVE_FP64, rb.LINKS_F64_12, 1e-8)])
 def test_same_bits_in_any_batch(torch_cuda, dims, mode, fmt, res):
@@ -67,3 +91,15 @@ def test_longer_than_one_launch(torch_cuda):
     assert ctx.true_residuals(xi, bi, SHIFTS * 1e-2).max() <= 20.0 * res  # iterated residual, kappa 4e5
     with pytest.raises(rb.RhmcError, match="cap 1030"):
         ctx.msolve_host(b, SHIFTS * 1e-2, res, max_iter=1030, mode=rb.MSOLVE_FP64, fmt=rb.LINKS_F64_18)
+
+
+def test_longer_than_one_launch_launch_by_launch(torch_cuda):
+    """The state that one launch of 1024 iterations leaves to the next."""
+    ctx, b = _case((8, 8, 8, 8), 0.004, 2, 71)
+    ctx.set_gauge(F.random_links((8, 8, 8, 8), seed=72))
+    out = []
+    for one in (1, 0):
+        ctx.msolve_one_kernel(one)
+        out.append(ctx.msolve_host(b, SHIFTS * 1e-2, 1e-7, mode=rb.MSOLVE_FP64, fmt=rb.LINKS_F64_18))
+    assert out[0][1]["iters"][0] > 1024 and out[0][1]["iters"] == out[1][1]["iters"]
+    assert np.array_equal(out[0][0], out[1][0])
