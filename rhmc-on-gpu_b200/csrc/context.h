@@ -131,6 +131,7 @@ struct rhmc_ctx {
     rhmc::Geom g;
     long V, Vh;
     int device;
+    int sms, l2_bytes;  // of the device
     double mass, beta;
     cudaStream_t stream;
     bool own_stream;

@@ -72,12 +72,12 @@ struct DslashArgs {
 // 24x20^2x18 1.15-1.24 times as fast with 18-real links and 2 or 4 right-hand sides, 24^3x32 1.05.
 // Where links and vectors stay in L2 between launches it only moves them between the two dies'
 // halves: 20^2x16x18 two right-hand sides (83 MB) 0.87, 18x14x16x22 eight (85 MB) 0.94, at 99 to
-// 110 MB neither, from 116 MB faster (L2: 126 MB).
+// 110 MB neither, from 116 MB faster, on an L2 of 132.6 MB (126.5 MiB).
 template <class LF, int NR>
-inline bool walk_alternates(long Vh)
+inline bool walk_alternates(long Vh, int l2_bytes)
 {
     const double bytes = (double)Vh * (8.0 * LF::bytes + 3.0 * NR * LF::store::planes * sizeof(typename LF::store::elem) / LF::store::pack);
-    return bytes > 105e6;
+    return bytes > 0.8 * l2_bytes;
 }
 
 // Re<y, o> of one colour added to a site's term of the fused reduction: FP64 products for FP64

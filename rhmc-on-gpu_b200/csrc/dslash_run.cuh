@@ -24,7 +24,7 @@ static cudaError_t run(rhmc_ctx *c, const LF &lf, int p_out, void *out, const vo
     a.stride = stride;
     a.alpha = (R)alpha;
     a.beta = (R)beta;
-    a.down = p_out == 0 && walk_alternates<LF, NR>(c->Vh);
+    a.down = p_out == 0 && walk_alternates<LF, NR>(c->Vh, c->l2_bytes);
     for (int r = 0; r < NR; r++) a.alphas[r] = (R)alpha;
     c->launches++;
     if (y) return dslash_launch<LF, NR, true, false, NoFin>(a, (int)c->Vh, c->stream);

@@ -14,8 +14,6 @@
 
 namespace rhmc {
 
-static int vec_grid(rhmc_ctx *c) { return grid_for(c->Vh, VEC_BLOCK); }
-
 int replay_until_stop(rhmc_ctx *c, cudaGraphExec_t exec, cudaStream_t s, const int *stop, long max_rep, long *replays,
                       int *stop_seen, const char *what)
 {
@@ -109,7 +107,7 @@ int true_residuals(rhmc_ctx *c, int nshift, const double *shifts, int nrhs, cons
     void *h, *t, *part;
     CK(c->ws.get("tr_h", 8 * stride * sizeof(double2), &h));
     CK(c->ws.get("tr_t", 8 * stride * sizeof(double2), &t));
-    const int gv = vec_grid(c);
+    const int gv = grid_for(c->Vh, VEC_BLOCK);
     CK(c->ws.get("tr_part", (size_t)gv * 8 * sizeof(double), &part));
     std::vector<double> hp((size_t)gv * 8);
     const int total = nrhs * nshift;

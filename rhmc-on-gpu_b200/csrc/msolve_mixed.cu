@@ -34,7 +34,6 @@
 
 namespace rhmc {
 
-constexpr int RB_MAX = 8;
 // iterations between reliable updates of the FP32 multi-shift phase
 constexpr int MX_RU_ITERS = 32;
 
@@ -108,7 +107,6 @@ int msolve_mixed(rhmc_ctx *c, int fmt, int nshift, const double *shifts, int nrh
     A.base = base.data();
     A.max_iter = max_iter;
     A.stop_on_frozen = 1;
-    A.chunk = 8;
     A.b = b;
     MSolveInfo mi;
     memset(&mi, 0, sizeof(mi));
@@ -225,7 +223,6 @@ static int msolve_fp64(rhmc_ctx *c, const rhmc_msolve_params *P, const double *s
         A.res_base = P->residual;
         A.max_iter = P->max_iter;
         A.stop_on_frozen = 1;
-        A.chunk = 8;
         A.b = b + (size_t)done * stride;
         A.x = x + (size_t)done * P->nshift * stride;
         MSolveInfo mi;
@@ -285,7 +282,6 @@ static int msolve_fp32(rhmc_ctx *c, const rhmc_msolve_params *P, const double *s
         A.res_base = P->residual;
         A.max_iter = P->max_iter;
         A.stop_on_frozen = 1;
-        A.chunk = 8;
         A.b = b + (size_t)done * stride;
         A.x = x + (size_t)done * P->nshift * stride;
         MSolveInfo mi;

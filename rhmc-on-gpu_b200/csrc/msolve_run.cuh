@@ -15,8 +15,6 @@
 
 namespace rhmc {
 
-static inline int vec_grid(rhmc_ctx *c) { return grid_for(c->Vh, VEC_BLOCK); }
-
 // workspace slot name of a base vector set in elements of `bytes` bytes
 static inline std::string vname(const char *base, size_t bytes) { return std::string(base) + std::to_string(bytes); }
 
@@ -123,7 +121,7 @@ static int ms_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *
     CK(c->ws.get(vname("ms_s", sizeof(E)), NR * vbytes, &s));
     CK(c->ws.get("ms_ps", (size_t)NR * S * v64, &ps));
     CK(c->ws.get("ms_state", sizeof(MSState), &stv));
-    const int gv = vec_grid(c);
+    const int gv = grid_for(Vh, VEC_BLOCK);
     CK(c->ws.get("ms_partials", (size_t)red_chunks(Vh) * 2 * NR * sizeof(double), &part));
     CK(c->ws.get("ms_tickets", 8 * sizeof(unsigned), &tick));
     // ring of the window's residuals [slot][rhs]
@@ -190,7 +188,7 @@ static int ms_phase(rhmc_ctx *c, const LF &lf, const MSolveArgs &A, MSolveInfo *
     a2.partials = pt;
     a2.ticket = tk + 1;
     a2.fin.st = st;
-    const int down = walk_alternates<LFB, NR>(Vh);
+    const int down = walk_alternates<LFB, NR>(Vh, c->l2_bytes);
     a2.down = down;
     a2.stop = &st->stop;
 

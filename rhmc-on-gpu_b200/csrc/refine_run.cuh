@@ -15,8 +15,6 @@
 
 namespace rhmc {
 
-constexpr int RB_MAX = 8;
-
 struct ResidCoef {
     double coef[8];  // mass^2 + sigma of each batched system
 };
@@ -312,7 +310,7 @@ static int rb_group(rhmc_ctx *c, const LF &lf, const double *coef, const double 
     s2.stride = sstride; s2.beta = (Rs)-0.5; s2.use_alphas = 1;
     for (int j = 0; j < NR; j++) s2.alphas[j] = (Rs)coef[j];
     s2.partials = pt; s2.ticket = tk + 1; s2.fin.st = st; s2.stop = &st->stop;
-    const int down = walk_alternates<LF, NR>(Vh);
+    const int down = walk_alternates<LF, NR>(Vh, c->l2_bytes);
     s2.down = down;
 
     struct Key {

@@ -329,7 +329,6 @@ struct F64S {
     typedef double real;
     typedef double2 elem;
     static constexpr int planes = 3;
-    static constexpr bool soa = true;  // plane c of site k at c * Vh + k
     static constexpr int pack = 1;    // right-hand sides per element (PackS)
     template <typename R>
     __device__ __forceinline__ static vec3<R> load(const elem *__restrict__ v, int Vh, int k)
@@ -348,24 +347,12 @@ struct F64S {
         for (int c = 0; c < 3; c++) d.c[c] = mk<double>((double)r.c[c].re, (double)r.c[c].im);
         store_spinor<double>(v, Vh, k, d);
     }
-    template <typename R>
-    __device__ __forceinline__ static vec3<R> load_plain(const elem *v, int pstride, int k)
-    {
-        vec3<R> r;
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            const elem a = v[c * pstride + k];
-            r.c[c] = mk<R>((R)a.x, (R)a.y);
-        }
-        return r;
-    }
 };
 
 struct F32S {
     typedef float real;
     typedef float2 elem;
     static constexpr int planes = 3;
-    static constexpr bool soa = true;
     static constexpr int pack = 1;
     template <typename R>
     __device__ __forceinline__ static vec3<R> load(const elem *__restrict__ v, int Vh, int k)
@@ -384,17 +371,6 @@ struct F32S {
         for (int c = 0; c < 3; c++) f.c[c] = mk<float>((float)r.c[c].re, (float)r.c[c].im);
         store_spinor<float>(v, Vh, k, f);
     }
-    template <typename R>
-    __device__ __forceinline__ static vec3<R> load_plain(const elem *v, int pstride, int k)
-    {
-        vec3<R> r;
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            const elem a = v[c * pstride + k];
-            r.c[c] = mk<R>((R)a.x, (R)a.y);
-        }
-        return r;
-    }
 };
 
 // The reference's host layout (Vec3 arrays, lib/Tools/vec3.h): the 3 complex numbers of a site
@@ -404,7 +380,6 @@ struct A64S {
     typedef double real;
     typedef double2 elem;
     static constexpr int planes = 3;
-    static constexpr bool soa = false;
     static constexpr int pack = 1;
     template <typename R>
     __device__ __forceinline__ static vec3<R> load(const elem *__restrict__ v, int, int k)
@@ -423,17 +398,6 @@ struct A64S {
 #pragma unroll
         for (int c = 0; c < 3; c++) v[(size_t)3 * k + c] = make_double2((double)r.c[c].re, (double)r.c[c].im);
     }
-    template <typename R>
-    __device__ __forceinline__ static vec3<R> load_plain(const elem *v, int, int k)
-    {
-        vec3<R> r;
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            const elem a = v[3 * k + c];
-            r.c[c] = mk<R>((R)a.x, (R)a.y);
-        }
-        return r;
-    }
 };
 
 // Half precision with a per-site scale, one 16-byte vector per site: words x, y, z hold the
@@ -444,7 +408,6 @@ struct H16S {
     typedef float real;
     typedef uint4 elem;
     static constexpr int planes = 1;
-    static constexpr bool soa = true;
     static constexpr int pack = 1;
     __device__ __forceinline__ static float2 h2f(unsigned w) { return __half22float2(*reinterpret_cast<const __half2 *>(&w)); }
     __device__ __forceinline__ static unsigned f2h(float a, float b)
@@ -590,7 +553,6 @@ struct PackS {
     typedef R real;
     typedef PackElem<R, P> elem;
     static constexpr int planes = 3;
-    static constexpr bool soa = true;
     static constexpr int pack = P;
 };
 

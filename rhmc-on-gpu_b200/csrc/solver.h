@@ -10,6 +10,8 @@ namespace rhmc {
 // from the last slot.
 __host__ __device__ inline int ms_prev_slot(int m, int win) { return m == 0 ? win - 1 : m - 1; }
 
+constexpr int RB_MAX = 8;  // systems of a refinement batch
+
 struct MSolveArgs {
     int nshift, nrhs;
     const double *shift;  // absolute shifts sigma_{r,i}, [nrhs][nshift] (each RHS its own pole set)
@@ -18,7 +20,6 @@ struct MSolveArgs {
     double res_base;      // stop when sqrt(|r|^2) <= res_base
     int max_iter;
     int stop_on_frozen;
-    int chunk;            // iterations per captured graph (the multi-shift loop uses its window, MS_WIN)
     const void *b;        // FP64 internal spinors, nrhs of them
     void *x;              // FP64 internal spinors, [nrhs][nshift]
     int fresh = 1;        // 1: start from x = 0; 0: resume the state an FP64 phase left (FP32 links only)

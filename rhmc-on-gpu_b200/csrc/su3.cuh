@@ -40,22 +40,6 @@ __device__ __forceinline__ M3 m3_mul(const M3 &a, const M3 &b)
     return r;
 }
 
-// a * b^dag
-__device__ __forceinline__ M3 m3_mul_nd(const M3 &a, const M3 &b)
-{
-    M3 r;
-#pragma unroll
-    for (int i = 0; i < 3; i++)
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-            C s = a.e[i][0] * conj(b.e[j][0]);
-            s = s + a.e[i][1] * conj(b.e[j][1]);
-            s = s + a.e[i][2] * conj(b.e[j][2]);
-            r.e[i][j] = s;
-        }
-    return r;
-}
-
 // a^dag * b
 __device__ __forceinline__ M3 m3_mul_dn(const M3 &a, const M3 &b)
 {
@@ -87,8 +71,6 @@ __device__ __forceinline__ void m3_scale(M3 &a, double s)
 #pragma unroll
         for (int j = 0; j < 3; j++) a.e[i][j] = s * a.e[i][j];
 }
-
-__device__ __forceinline__ double m3_retr(const M3 &a) { return a.e[0][0].re + a.e[1][1].re + a.e[2][2].re; }
 
 // a b^* + c in four FMAs (a product formed first and then added costs two more operations)
 __device__ __forceinline__ C cmaddc(C a, C b, C c)

@@ -225,7 +225,7 @@ int link_update(rhmc_ctx *c, double step)
 int plaquette_sums(rhmc_ctx *c, double *temporal, double *spatial)
 {
     const int sites = grid_for(2L * grid_for(c->Vh, 32), PLAQ_BLOCK / 32);  // blocks; a warp per 32 half-sites
-    const int split = sites <= PLAQ_RESIDENT * 148 ? 6 : 1;
+    const int split = sites <= PLAQ_RESIDENT * c->sms ? 6 : 1;
     const int nb = sites * split;
     void *part;
     CK(c->ws.get("red_part", (size_t)nb * 2 * sizeof(double), &part));
