@@ -102,7 +102,7 @@ __host__ __device__ __forceinline__ long force_chunks(int Vh, int W) { return 2L
 // link-plane load of the warp is one contiguous 512-byte segment (own links) or nearly so
 // (neighbour links).  The four warps of a block are the four mu of one chunk: of the 76 links they
 // load per site 44 are distinct, and the repeats hit L1 (with mu as the slow index the whole link
-// field was streamed from HBM once per mu).  Bound by FP64 issue (52 %) and L2 latency together:
+// field was streamed from HBM once per mu).  Bound by FP64 issue (59 % of its rate) and L2 latency together:
 // 1,450 FP64 instructions and 19 link loads per link at the 12 warps per SM that 168 registers
 // allow.  32^4: 605 us; 755 us when the products were formed with separate additions (1,900 FP64
 // instructions), 616 us with mu as the fastest block index; 658 us at 16 warps and 128 registers,
